@@ -10,6 +10,7 @@
 #include "fwd_alt_sm100.cuh"
 #include "fwd_one_sm100.cuh"
 #include "fwd_pers_sm100.cuh"
+#include "fwd_split_sm100.cuh"
 
 namespace fray {
 
@@ -24,6 +25,8 @@ enum AttnKernelKind : int {
                              // two CTAs per SM cover each other's start, end and softmax phases
   kAttnPersistent = 5,       // kind 1 as one CTA per SM that walks through the work items, the next item's first
                              // copies and scores behind the current item's last steps
+  kAttnFewQueries = 6,       // all rows of a K/V head's group in one tile, keys split over a cluster of CTAs; what does
+                             // not have that form runs as kind 1
 };
 
 // KIND, D, BLOCK_N, STAGES are compile-time tuning keys (BLOCK_N: KV tile of the single-role kernel, 128
@@ -60,6 +63,12 @@ inline void flash_attn_sm100(const operand_t* q, const operand_t* k, const opera
     rc = sm100::launch_attn_fwd_one<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
   } else if constexpr (KIND == kAttnPersistent) {
     rc = sm100::launch_attn_fwd_pers<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
+  } else if constexpr (KIND == kAttnFewQueries) {
+    if (sm100::split_applies(shp, ex, causal)) {
+      rc = sm100::launch_attn_fwd_split<D>(q, k, v, o, shp, st, ex, scale, stream);
+    } else {
+      rc = sm100::launch_attn_fwd_ws<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
+    }
   } else {
     static_assert(KIND == kAttnPaired, "unknown kernel kind");
     static_assert(D == 128, "the paired kernel is built for head dim 128");

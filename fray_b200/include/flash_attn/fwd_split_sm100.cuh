@@ -1,0 +1,468 @@
+#pragma once
+// Few-query attention forward for sm_100a: at most 128 (query, head-of-group) rows per K/V head, any number of keys.
+//
+// A decoding step or a short chunk of new queries against a long cache reads every key and value once and does
+// little arithmetic: the copies bound it (8 x 8 K/V heads x 8192 keys x 128 bf16: 268 MB, 41 us at the measured copy
+// rate), and one CTA per query head would read them once per head of a group and leave most of the chip idle.
+//
+//   * all query heads of a K/V head's group share one CTA's tile: row = head_in_group * seq_q + query, fetched by one
+//     copy whose box spans the group's heads;
+//   * the keys of a (batch, K/V head) unit are cut into `splits` runs of 128-key tiles, one CTA each; the CTAs of a
+//     unit form a cluster and merge their partial results through each other's shared memory, so there is no
+//     workspace, no second launch and no order between clusters;
+//   * a tile of up to 32 rows is placed four times (up to 64: twice) in the 128-row operand, and the warps, each of which
+//     reaches only its own 32 lanes of tensor memory, each take a quarter (half) of a step's keys for the same rows: the
+//     P of the other keys stays zero, the copies' partial sums are merged with the splits'.  The warps share nothing
+//     inside a step, and a step's exponentials take a quarter of the time;
+//   * scores and probabilities have two tensor-memory buffers each, so S(t+2) is issued behind P.V(t) and the
+//     tensor pipe never waits for a softmax of its own step.
+//
+// Measured (device time, back to back on three sets of buffers): 8 x 8 K/V heads x 8192 keys x 128 bf16, 4 query heads
+// each 43.6 us = 6.2 TB/s (one 128-row tile per query head: 124 us); 1 x 8 x 16384 18.7 us (206 us); 16 x 8 x 16384 with
+// 8 query heads each 160 us (1020 us); 2 x 8 heads x 100 queries x 2000 keys 14.5 us (31 us).
+//
+// Warps 0-3 softmax and epilogue, warp 4 MMA issue, warp 5 TMA producer, warps 6-7 help with the merge.
+// Every barrier wait is bounded (see sm100_ptx.cuh).
+
+#include "host_sm100.cuh"
+#include "sm100_ptx.cuh"
+#include "softmax_tile_sm100.cuh"
+
+namespace fray {
+namespace sm100 {
+
+template <int D>
+struct SplitCfg {
+  static constexpr int BM = 128, BN = 128;
+  static constexpr int kThreads = 256;
+  static constexpr int kStages = D == 128 ? 6 : 12;
+  static constexpr int kPanels = D / 64;
+  static constexpr int kQPanelBytes = BM * 128;
+  static constexpr int kQTileBytes = kPanels * kQPanelBytes;
+  static constexpr int kKVPanelBytes = BN * 128;
+  static constexpr int kKVTileBytes = kPanels * kKVPanelBytes;
+  static constexpr int kOffKV = kQTileBytes;
+  static constexpr int kPartStride = D + 4;  // floats from row to row of the partial results (they take the ring's place)
+  static_assert(BM * kPartStride * 4 <= kStages * kKVTileBytes, "the partial results fit the ring");
+  static constexpr int kOffBars = kOffKV + kStages * kKVTileBytes;
+  static constexpr int kNumBars = 1 + 2 * kStages + 5;
+  static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // (m, l) per partial row
+  static constexpr int kSmemBytes = kOffStats + BM * 8 + 1024;
+  static_assert(kSmemBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
+  static constexpr int kTmemCols = 512;
+  static constexpr uint32_t kColS = 0, kColP = 256, kColO = 384;  // S(t) at 128 * (t & 1), P(t) at 256 + 64 * (t & 1)
+  static constexpr int kMaxSplits = 8;                           // portable cluster size
+};
+
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
+// COPIES: how often the rows are placed in the 128-row operand (4 up to 32 rows, 2 up to 64, 1 up to 128).
+template <int D, int COPIES>
+__global__ void __launch_bounds__(256, 1)
+attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, operand_t* o, long long o_sb, long long o_sh, long long o_ss,
+                      int num_kv_heads, int group, int seq_q, float scale_log2, float* lse, int seq_k) {
+  using Cfg = SplitCfg<D>;
+  constexpr int BN = Cfg::BN, STAGES = Cfg::kStages;
+  constexpr int kRowsPerCopy = Cfg::BM / COPIES;
+  constexpr int NCH = 4 / COPIES;  // chunks of 32 keys a warp takes of every step
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint8_t* q_smem = smem;
+  uint8_t* kv_smem = smem + Cfg::kOffKV;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
+  uint64_t* q_full = bars;
+  uint64_t* kv_full = bars + 1;
+  uint64_t* kv_empty = kv_full + STAGES;
+  uint64_t* s_full = kv_empty + STAGES;  // [2] MMA -> softmax (S(t), buffer t & 1)
+  uint64_t* p_full = s_full + 2;         // [2] softmax -> MMA (P(t), buffer t & 1)
+  uint64_t* o_full = p_full + 2;         // MMA -> softmax (P.V(t) complete)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
+  float2* part_ml = reinterpret_cast<float2*>(smem + Cfg::kOffStats);
+  float* part_o = reinterpret_cast<float*>(kv_smem);
+
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  const int splits = gridDim.x, split = blockIdx.x;  // the cluster spans the x axis
+  const int b = blockIdx.y / num_kv_heads;
+  const int h_kv = blockIdx.y - b * num_kv_heads;
+  const int rows = group * seq_q;
+  const int n_kv = (seq_k + BN - 1) / BN;
+  const int t_first = static_cast<int>(static_cast<long long>(n_kv) * split / splits);
+  const int t_last = static_cast<int>(static_cast<long long>(n_kv) * (split + 1) / splits);
+
+  if (tid == 0) {
+    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
+    mbar_init(q_full, 1);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(kv_full + s, 1);
+      mbar_init(kv_empty + s, 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(s_full + 1, 1);
+    mbar_init(p_full, 4);
+    mbar_init(p_full + 1, 4);
+    mbar_init(o_full, 1);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  // An earlier launch left the device status raised: compute nothing, but meet the cluster's barriers.
+  const bool dead = *abort_flag != 0;
+  const int n = dead ? 0 : t_last - t_first;
+
+  if (warp < 4) {
+    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    const int c0 = (warp * COPIES / 4) * NCH;  // this warp's first chunk of 32 keys
+    const uint32_t t_o = tmem_base + Cfg::kColO + lane_base;
+    const int slot = warp * 32 + lane;
+    const bool mine = slot % kRowsPerCopy < rows;  // the other lanes' rows hold whatever shared memory held
+    if (COPIES > 1) {  // P of the keys other copies take: zero, and nothing writes there again
+      uint32_t z[16];
+#pragma unroll
+      for (int x = 0; x < 16; ++x) z[x] = 0u;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) tmem_st_x16(tmem_base + Cfg::kColP + c * 16 + lane_base, z);
+      tmem_wait_st();
+    }
+    float m_ref = -INFINITY, l_run = 0.f;
+    for (int t = 0; t < n; ++t) {
+      const uint32_t t_s = tmem_base + Cfg::kColS + (t & 1) * 128 + lane_base;
+      const uint32_t t_p = tmem_base + Cfg::kColP + (t & 1) * 64 + lane_base;
+      mbar_wait(s_full + (t & 1), (t >> 1) & 1, abort_flag, 0x201, t);
+      tc_fence_after_sync();
+      uint32_t s[NCH][32];
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) tmem_ld_x32(t_s + (c0 + c) * 32, s[c]);
+      tmem_wait_ld();
+      const int lim = seq_k - (t_first + t) * BN - c0 * 32;  // keys of this warp's part that exist
+      if (lim < NCH * 32) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+#pragma unroll
+          for (int x = 0; x < 32; ++x)
+            if (c * 32 + x >= lim) s[c][x] = __float_as_uint(-INFINITY);
+      }
+      float mx0 = m_ref, mx1 = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c)
+#pragma unroll
+        for (int x = 0; x < 32; x += 4) {
+          mx0 = max3(mx0, __uint_as_float(s[c][x]), __uint_as_float(s[c][x + 1]));
+          mx1 = max3(mx1, __uint_as_float(s[c][x + 2]), __uint_as_float(s[c][x + 3]));
+        }
+      const float m_new = fmaxf(mx0, mx1);
+      if (t == 0) {
+        m_ref = m_new;
+      } else {
+        float alpha = 1.f;
+        if (mine && (m_new - m_ref) * scale_log2 > kRescaleThreshold) {
+          alpha = ex2_approx((m_ref - m_new) * scale_log2);
+          l_run *= alpha;
+          m_ref = m_new;
+        }
+        if (__any_sync(0xffffffffu, alpha != 1.f)) {
+          mbar_wait(o_full, (t - 1) & 1, abort_flag, 0x311, t);  // the previous P.V has landed in O
+          tc_fence_after_sync();
+#pragma unroll 1
+          for (int c = 0; c < D; c += 16) {
+            uint32_t orr[16];
+            tmem_ld_x16(t_o + c, orr);
+            tmem_wait_ld();
+#pragma unroll
+            for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+            tmem_st_x16(t_o + c, orr);
+          }
+        }
+      }
+      const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * scale_log2;
+      uint64_t rsp0 = 0ull, rsp1 = 0ull;
+      const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2), neg_m2 = pack_f32x2(neg_m, neg_m);
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        uint32_t pk[16];
+        exp_32(s[c], scale2, neg_m2, rsp0, rsp1, pk);
+        tmem_st_x16(t_p + (c0 + c) * 16, pk);
+      }
+      tmem_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full + (t & 1));
+      float r0, r1, r2, r3;
+      unpack_f32x2(rsp0, r0, r1);
+      unpack_f32x2(rsp1, r2, r3);
+      l_run += (r0 + r1) + (r2 + r3);
+    }
+    if (n > 0) {
+      // S(n-1) may be complete before P.V(n-2) is: pass that phase first, or the last one's parity would look over
+      if (n > 1) mbar_wait(o_full, (n - 2) & 1, abort_flag, 0x330, n);
+      mbar_wait(o_full, (n - 1) & 1, abort_flag, 0x331, n);
+      tc_fence_after_sync();
+      // Every copy into the ring has been read by a completed product: the partial results take its place.
+#pragma unroll
+      for (int c = 0; c < D; c += 32) {
+        uint32_t orr[32];
+        tmem_ld_x32(t_o + c, orr);
+        tmem_wait_ld();
+        if (mine) {
+#pragma unroll
+          for (int x = 0; x < 32; x += 4)
+            *reinterpret_cast<uint4*>(part_o + slot * Cfg::kPartStride + c + x) = make_uint4(orr[x], orr[x + 1], orr[x + 2], orr[x + 3]);
+        }
+      }
+      if (mine) part_ml[slot] = make_float2(m_ref, l_run);
+    }
+  } else if (warp == 5 && lane == 0) {
+    // ============================================================= TMA producer
+    if (n > 0) {
+      mbar_expect_tx(q_full, COPIES * rows * 128 * Cfg::kPanels);
+#pragma unroll
+      for (int cp = 0; cp < COPIES; ++cp)
+#pragma unroll
+        for (int p = 0; p < Cfg::kPanels; ++p)
+          tma_load_4d(q_smem + p * Cfg::kQPanelBytes + cp * kRowsPerCopy * 128, &tm_q, q_full, p * 64, 0, h_kv * group, b);
+    }
+    uint32_t c = 0;
+    auto load = [&](const CUtensorMap* tm, int t) __attribute__((always_inline)) {
+      const int slot = c % STAGES;
+      mbar_wait(kv_empty + slot, ((c / STAGES) & 1) ^ 1, abort_flag, 0x401, t);
+      if (*abort_flag != 0) return;
+      mbar_expect_tx(kv_full + slot, Cfg::kKVTileBytes);
+#pragma unroll
+      for (int p = 0; p < Cfg::kPanels; ++p)
+        tma_load_4d(kv_smem + slot * Cfg::kKVTileBytes + p * Cfg::kKVPanelBytes, tm, kv_full + slot, p * 64,
+                    (t_first + t) * BN, h_kv, b);
+      ++c;
+    };
+    // in the order the products read them: K0 K1 V0 K2 V1 ...
+    if (n > 0) load(&tm_k, 0);
+    for (int t = 0; t < n; ++t) {
+      if (t + 1 < n) load(&tm_k, t + 1);
+      load(&tm_v, t);
+      if (*abort_flag != 0) break;
+    }
+  } else if (warp == 4) {
+    // ============================================================= MMA issue (whole warp, one elected lane issues)
+    constexpr uint64_t kDescK = smem_desc_sw128(16, 1024);
+    constexpr uint64_t kDescV = smem_desc_sw128(Cfg::kKVPanelBytes, 1024);
+    constexpr uint32_t kIdescQK = idesc_f16_f32(Cfg::BM, BN, false, false);
+    constexpr uint32_t kIdescPV = idesc_f16_f32(Cfg::BM, D, false, true);
+    constexpr uint32_t kDescHi = static_cast<uint32_t>(kDescK >> 32), kDescLo = static_cast<uint32_t>(kDescK);
+    constexpr uint32_t kDescVHi = static_cast<uint32_t>(kDescV >> 32);
+    const uint32_t kv_addr = smem_u32(kv_smem);
+    const uint32_t q_lo = kDescLo | ((smem_u32(q_smem) & 0x3FFFF) >> 4);
+    uint32_t c = 0;
+    auto issue_qk = [&](int t) __attribute__((always_inline)) {
+      const int slot = c % STAGES;
+      mbar_wait(kv_full + slot, (c / STAGES) & 1, abort_flag, 0x501, t);
+      tc_fence_after_sync();
+      const uint32_t k_lo = kDescLo | (((kv_addr + slot * Cfg::kKVTileBytes) & 0x3FFFF) >> 4);
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t qoff = ((kk >> 2) * Cfg::kQPanelBytes + (kk & 3) * 32) >> 4;
+        const uint32_t koff = ((kk >> 2) * Cfg::kKVPanelBytes + (kk & 3) * 32) >> 4;
+        mma_ss_elect_lohi(tmem_base + Cfg::kColS + (t & 1) * 128, q_lo + qoff, kDescHi, k_lo + koff, kDescHi, kIdescQK, kk > 0);
+      }
+      mma_commit_elect(s_full + (t & 1));
+      mma_commit_elect(kv_empty + slot);
+      ++c;
+    };
+    auto issue_pv = [&](int t) __attribute__((always_inline)) {
+      const int slot = c % STAGES;
+      mbar_wait(kv_full + slot, (c / STAGES) & 1, abort_flag, 0x502, t);
+      mbar_wait(p_full + (t & 1), (t >> 1) & 1, abort_flag, 0x503, t);
+      tc_fence_after_sync();
+      const uint32_t v_lo = static_cast<uint32_t>(kDescV) | (((kv_addr + slot * Cfg::kKVTileBytes) & 0x3FFFF) >> 4);
+#pragma unroll
+      for (int kk = 0; kk < BN / 16; ++kk)
+        mma_ts_elect_lohi(tmem_base + Cfg::kColO, tmem_base + Cfg::kColP + (t & 1) * 64 + kk * 8, v_lo + ((kk * 2048) >> 4),
+                          kDescVHi, kIdescPV, (t > 0 || kk > 0));
+      mma_commit_elect(o_full);
+      mma_commit_elect(kv_empty + slot);
+      ++c;
+    };
+    if (n > 0) {
+      mbar_wait(q_full, 0, abort_flag, 0x511);
+      issue_qk(0);
+    }
+    for (int t = 0; t < n; ++t) {
+      if (t + 1 < n) issue_qk(t + 1);
+      issue_pv(t);
+    }
+  }
+
+  // Merge: every CTA of the cluster adds up a share of the outputs over all partial results.
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  __syncwarp();
+  cluster_sync_all();
+  if (!dead) {
+    const uint32_t o_addr = smem_u32(part_o), ml_addr = smem_u32(part_ml);
+    const int total = rows * (D / 4);
+    for (int e = split * Cfg::kThreads + tid; e < total; e += splits * Cfg::kThreads) {
+      const int r = e / (D / 4), c4 = e - r * (D / 4);
+      float m = -INFINITY, l = 0.f;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      // Several CTAs' results are fetched at a time: one load from another SM takes some hundred cycles.
+      constexpr int kAtOnce = 4 / COPIES;
+      for (int p0 = 0; p0 < splits; p0 += kAtOnce) {
+        float2 ml[4];
+        float4 v[4];
+#pragma unroll
+        for (int a = 0; a < kAtOnce; ++a) {
+          const int p = p0 + a < splits ? p0 + a : splits - 1;
+          const uint32_t po = mapa_shared(o_addr, p), pm = mapa_shared(ml_addr, p);
+#pragma unroll
+          for (int cp = 0; cp < COPIES; ++cp) {
+            ml[a * COPIES + cp] = ld_cluster_f2(pm + (cp * kRowsPerCopy + r) * 8);
+            v[a * COPIES + cp] = ld_cluster_f4(po + ((cp * kRowsPerCopy + r) * Cfg::kPartStride + c4 * 4) * 4);
+          }
+        }
+        float m_all = m;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) m_all = fmaxf(m_all, ml[x].x);
+        const float m_safe = m_all == -INFINITY ? 0.f : m_all;  // no key so far: every weight is 0
+        const float w0 = ex2_approx((m - m_safe) * scale_log2);
+        l *= w0;
+        acc.x *= w0; acc.y *= w0; acc.z *= w0; acc.w *= w0;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          if (p0 + x / COPIES < splits) {
+            const float w = ex2_approx((ml[x].x - m_safe) * scale_log2);
+            l += ml[x].y * w;
+            acc.x += v[x].x * w; acc.y += v[x].y * w; acc.z += v[x].z * w; acc.w += v[x].w * w;
+          }
+        }
+        m = m_all;
+      }
+      const float inv_l = l > 0.f ? 1.f / l : 1.f;
+      const int g = r / seq_q, s = r - g * seq_q;
+      const int h = h_kv * group + g;
+      *reinterpret_cast<uint2*>(o + b * o_sb + h * o_sh + s * o_ss + c4 * 4) =
+          make_uint2(pack_half2(acc.x * inv_l, acc.y * inv_l), pack_half2(acc.z * inv_l, acc.w * inv_l));
+      if (lse != nullptr && c4 == 0)
+        lse[(static_cast<size_t>(b) * num_kv_heads * group + h) * seq_q + s] =
+            l > 0.f ? (m * scale_log2 + log2f(l)) * 0.69314718055994531f : -INFINITY;
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // shared memory stays until every CTA has read it
+}
+
+// CTAs per (batch, K/V head) unit: the cluster size that needs the fewest rounds of tiles, counting three tiles' time
+// for a CTA's start, merge and end.  active[c]: clusters of c CTAs that run at the same time.  That is not SMs / c: a
+// cluster lives in one GPC, and 16 units x 1024 keys as 16 clusters of 8 (128 CTAs on 148 SMs) took two rounds, 18.0 us
+// against 10.6 us as clusters of fewer CTAs in one round.
+inline int split_count(int units, int n_kv, const int (&active)[SplitCfg<128>::kMaxSplits + 1]) {
+  int best = 1;
+  long long best_cost = -1;
+  for (int c = 1; c <= SplitCfg<128>::kMaxSplits && c <= n_kv; ++c) {
+    const long long rounds = (static_cast<long long>(units) + active[c] - 1) / active[c];
+    const long long cost = rounds * ((n_kv + c - 1) / c + 3);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = c;
+    }
+  }
+  return best;
+}
+
+// True when the problem has the form this kernel is written for.
+inline bool split_applies(const AttnShape& shp, const AttnExtras& ex, bool causal) {
+  return !causal && static_cast<long long>(ex.kv_group) * shp.S <= 128;
+}
+
+template <int D, int COPIES>
+inline int launch_attn_fwd_split_copies(const operand_t* q, const operand_t* k, const operand_t* v, operand_t* o,
+                                        const AttnShape& shp, const AttnStrides (&st)[4], const AttnExtras& ex, float scale,
+                                        cudaStream_t stream) {
+  using Cfg = SplitCfg<D>;
+  struct Tag {};
+  const AttnShape shp_kv{shp.B, shp.H / ex.kv_group, ex.seq_k, shp.D};
+  CUtensorMap tm_q, tm_k, tm_v;
+  int rc = cached_attn_tensor_map(&tm_q, q, shp, st[0], shp.S, ex.kv_group);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_k, k, shp_kv, st[1], Cfg::BN);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_v, v, shp_kv, st[2], Cfg::BN);
+  if (rc != kAttnOk) return rc;
+  auto kernel = attn_fwd_split_kernel<D, COPIES>;
+  rc = ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes);
+  if (rc != kAttnOk) return rc;
+  const int units = shp_kv.B * shp_kv.H;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(Cfg::kThreads);
+  cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  auto clusters_of = [&](int c) {
+    cfg.gridDim = dim3(c, units);
+    attr[0].val.clusterDim.x = c;
+  };
+  // how many clusters of each size the device runs at a time: asked once per host thread and device
+  thread_local int active[Cfg::kMaxSplits + 1] = {};
+  thread_local int active_dev = -1;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return kAttnLaunchFailed;
+  }
+  if (dev != active_dev) {
+    for (int c = 1; c <= Cfg::kMaxSplits; ++c) {
+      clusters_of(c);
+      if (cudaOccupancyMaxActiveClusters(&active[c], kernel, &cfg) != cudaSuccess || active[c] <= 0) {
+        (void)cudaGetLastError();
+        return kAttnLaunchFailed;
+      }
+    }
+    active_dev = dev;
+  }
+  clusters_of(split_count(units, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, active));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_q, tm_k, tm_v, o, static_cast<long long>(shp.B > 1 ? st[3].b : 0),
+                                           static_cast<long long>(shp.H > 1 ? st[3].h : 0),
+                                           static_cast<long long>(shp.S > 1 ? st[3].s : 0), shp_kv.H, ex.kv_group, shp.S,
+                                           scale * 1.44269504088896340736f, ex.lse, ex.seq_k);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return kAttnLaunchFailed;
+  }
+  return kAttnOk;
+}
+
+// Host launcher for the few-query kernel. Returns an AttnReturnCode.
+template <int D>
+inline int launch_attn_fwd_split(const operand_t* q, const operand_t* k, const operand_t* v, operand_t* o, const AttnShape& shp,
+                                 const AttnStrides (&st)[4], const AttnExtras& ex, float scale, cudaStream_t stream) {
+  const int rows = ex.kv_group * shp.S;
+  if (rows <= 32) return launch_attn_fwd_split_copies<D, 4>(q, k, v, o, shp, st, ex, scale, stream);
+  if (rows <= 64) return launch_attn_fwd_split_copies<D, 2>(q, k, v, o, shp, st, ex, scale, stream);
+  return launch_attn_fwd_split_copies<D, 1>(q, k, v, o, shp, st, ex, scale, stream);
+}
+
+}  // namespace sm100
+}  // namespace fray

@@ -83,9 +83,9 @@ inline PFN_encodeTiled get_encode_tiled() {
 }
 
 // Tensor map over a 16-bit (fp16 or bf16, see operand_t) [B,H,S,D] tensor (D contiguous) whose box is
-// `box_rows` sequence positions x 64 head-dim elements (one 128-byte swizzle span).
+// `box_heads` heads x `box_rows` sequence positions x 64 head-dim elements (one 128-byte swizzle span).
 inline int make_attn_tensor_map(CUtensorMap* map, const void* base, const AttnShape& shp, const AttnStrides& st,
-                                int box_rows) {
+                                int box_rows, int box_heads) {
   PFN_encodeTiled enc = get_encode_tiled();
   if (enc == nullptr) return kAttnNoDriverEntry;
   // A size-1 mode never advances, so any legal (16-byte multiple) stride will do.
@@ -96,7 +96,7 @@ inline int make_attn_tensor_map(CUtensorMap* map, const void* base, const AttnSh
                         static_cast<cuuint64_t>(shp.H), static_cast<cuuint64_t>(shp.B)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(ss) * 2, static_cast<cuuint64_t>(sh) * 2,
                            static_cast<cuuint64_t>(sb) * 2};
-  cuuint32_t box[4] = {64u, static_cast<cuuint32_t>(box_rows), 1u, 1u};
+  cuuint32_t box[4] = {64u, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_heads), 1u};
   cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   CUresult r = enc(map, kOperandIsBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -108,12 +108,12 @@ inline int make_attn_tensor_map(CUtensorMap* map, const void* base, const AttnSh
 // launches on the same buffers again (the common case: a fixed set of activations per layer, or a
 // benchmark loop) skips the driver call.  A tensor map depends only on the key compared below.
 inline int cached_attn_tensor_map(CUtensorMap* map, const void* base, const AttnShape& shp, const AttnStrides& st,
-                                  int box_rows) {
+                                  int box_rows, int box_heads = 1) {
   struct Entry {
     const void* base = nullptr;
     AttnShape shp{0, 0, 0, 0};
     AttnStrides st{0, 0, 0};
-    int box_rows = 0;
+    int box_rows = 0, box_heads = 0;
     CUtensorMap map;
   };
   constexpr int kEntries = 16;
@@ -121,13 +121,13 @@ inline int cached_attn_tensor_map(CUtensorMap* map, const void* base, const Attn
   thread_local int next = 0;
   for (int e = 0; e < kEntries; ++e) {
     const Entry& c = cache[e];
-    if (c.base == base && c.box_rows == box_rows && c.shp.B == shp.B && c.shp.H == shp.H && c.shp.S == shp.S &&
+    if (c.base == base && c.box_rows == box_rows && c.box_heads == box_heads && c.shp.B == shp.B && c.shp.H == shp.H && c.shp.S == shp.S &&
         c.shp.D == shp.D && c.st.b == st.b && c.st.h == st.h && c.st.s == st.s) {
       *map = c.map;
       return kAttnOk;
     }
   }
-  const int rc = make_attn_tensor_map(map, base, shp, st, box_rows);
+  const int rc = make_attn_tensor_map(map, base, shp, st, box_rows, box_heads);
   if (rc == kAttnOk) {
     Entry& c = cache[next];
     next = (next + 1) % kEntries;
@@ -135,6 +135,7 @@ inline int cached_attn_tensor_map(CUtensorMap* map, const void* base, const Attn
     c.shp = shp;
     c.st = st;
     c.box_rows = box_rows;
+    c.box_heads = box_heads;
     c.map = *map;
   }
   return rc;

@@ -78,6 +78,31 @@ inline int read_attn_trace(unsigned int* out, int max_words) {
 // Lazy-rescale threshold in the scaled base-2 domain: offsets move only when the max grew by > 2^8.
 static constexpr float kRescaleThreshold = 8.0f;
 
+// 32 keys of one row: exponentials in base 2 of scale * score - offset, row sum from the unrounded values (two packed
+// partial sums), rounding to 16 bits.
+__device__ __forceinline__ void exp_32(const uint32_t (&h)[32], uint64_t scale2, uint64_t neg_m2, uint64_t& rsp0,
+                                       uint64_t& rsp1, uint32_t (&pk)[16]) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 8) {
+    uint64_t p[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(h[c + 2 * e]), __uint_as_float(h[c + 2 * e + 1])), scale2, neg_m2);
+      float x0, x1;
+      unpack_f32x2(x, x0, x1);
+      p[e] = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
+    }
+    rsp0 = add_f32x2(rsp0, add_f32x2(p[0], p[2]));
+    rsp1 = add_f32x2(rsp1, add_f32x2(p[1], p[3]));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float p0, p1;
+      unpack_f32x2(p[e], p0, p1);
+      pk[(c >> 1) + e] = pack_half2(p0, p1);
+    }
+  }
+}
+
 // t_s        tensor-memory address of this thread's lane at column 0 of the S tile (P overwrites it)
 // p_bar      PCHUNKS consecutive mbarriers, arrival count 4 (one per warp of the group): chunk q of P stored
 // rescale_o  called by every thread with the factor its row of O has to be multiplied by before this

@@ -76,6 +76,31 @@ _RC_TENSOR_MAP = 6
 
 # Kernel kinds (flash_attn/flash_attn_sm100.cuh).
 KIND_SIMPLE, KIND_TWO_TILES, KIND_ALTERNATING, KIND_PAIRED, KIND_ONE_TILE, KIND_PERSISTENT = 0, 1, 2, 3, 4, 5
+KIND_FEW_QUERIES = 6
+
+# The few-query kernel holds all rows (queries x query heads per K/V head) of a K/V head in one 128-row tile.
+FEW_QUERY_ROWS = 128
+# Below this many keys its cluster's start and merge cost more than the split saves (16 heads x 128 queries, head dim
+# 128: 11.2 us against 7.3 at 256 keys, 9.5 against 10.8 at 512, 10.6 against 17.2 at 1024).
+FEW_QUERY_MIN_KEYS = 512
+# With a K/V head per query head there are no rows to share, and once the units fill the chip by themselves only long
+# units gain (1024 units: 61 us against 51 at 512 keys, 92 against 90 at 1024, 185 against 228 at 4096).
+FEW_QUERY_LONG_KEYS = 4096
+
+
+def few_query_space() -> Tuple[Dict[str, Any], ...]:
+    """The one kernel for calls of few queries (see ``_few_queries``); BLOCK_N and STAGES are those of the two-tile
+    kernel its library falls back to."""
+    return ({"KIND": KIND_FEW_QUERIES, "BLOCK_N": 128, "STAGES": 4},)
+
+
+def _few_queries(group: int, seq_len: int, seq_len_kv: int, causal: bool, units: int, sms: int) -> bool:
+    """Whether a call goes to the few-query kernel: all rows of a K/V head's group fit one tile, every row sees every
+    key and there are many keys (a decoding step, a short chunk of new queries).  Such a call is bound by reading K and V
+    once, not by arithmetic.  ``units``: batch x K/V heads."""
+    if causal or group * seq_len > FEW_QUERY_ROWS or seq_len_kv < FEW_QUERY_MIN_KEYS:
+        return False
+    return group > 1 or units <= sms or seq_len_kv >= FEW_QUERY_LONG_KEYS
 
 
 def tuning_space(d: int) -> Tuple[Dict[str, Any], ...]:
@@ -140,7 +165,8 @@ def _space_points(head_dims, forced: bool):
     """(d, point, bf16) for every library of the tuning space (forced: honour FRAY_ATTN_FORCE)."""
     old = None if forced else os.environ.pop("FRAY_ATTN_FORCE", None)
     try:
-        return [(d, point, bf16) for d in head_dims for bf16 in (False, True) for point in tuning_space(d)]
+        few = () if forced else few_query_space()
+        return [(d, point, bf16) for d in head_dims for bf16 in (False, True) for point in (*tuning_space(d), *few)]
     finally:
         if old is not None:
             os.environ["FRAY_ATTN_FORCE"] = old
@@ -283,11 +309,14 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
 
     args = pack(q, k, v, out)
     forced = os.getenv("FRAY_ATTN_FORCE", "")
+    few = not forced and _few_queries(num_heads // num_kv_heads, seq_len, seq_len_kv, bool(causal), batch_size * num_kv_heads,
+                                           torch.cuda.get_device_properties(Q.device).multi_processor_count)
     runtime = jit_tuner.compile_and_tune(
         name="flash_attn_cute",
-        keys={"D": d, "CAUSAL": int(bool(causal)), "CLASS": _seq_class(max(seq_len, seq_len_kv), batch_size * num_heads),
+        keys={"D": d, "CAUSAL": int(bool(causal)),
+              "CLASS": "few" if few else _seq_class(max(seq_len, seq_len_kv), batch_size * num_heads),
               "FORCED": forced, **({"BF16": 1} if bf16 else {})},
-        space=tuning_space(d),
+        space=few_query_space() if few else tuning_space(d),
         includes=includes_bf16 if bf16 else includes,
         arg_defs=arg_defs_bf16 if bf16 else arg_defs,
         template=template,
