@@ -9,7 +9,7 @@
 #include "fwd_ws_sm100.cuh"
 #include "fwd_alt_sm100.cuh"
 #include "fwd_one_sm100.cuh"
-#include "fwd_pers_sm100.cuh"
+#include "fwd_duo_sm100.cuh"
 #include "fwd_split_sm100.cuh"
 
 namespace fray {
@@ -23,10 +23,10 @@ enum AttnKernelKind : int {
   kAttnPaired = 3,           // the same on a pair of CTAs (cta_group::2): 256 rows per pair, half of K and V per CTA
   kAttnOneTile = 4,          // one 128-row tile per CTA, producer / MMA / softmax roles, 256 tensor-memory columns:
                              // two CTAs per SM cover each other's start, end and softmax phases
-  kAttnPersistent = 5,       // kind 1 as one CTA per SM that walks through the work items, the next item's first
-                             // copies and scores behind the current item's last steps
   kAttnFewQueries = 6,       // all rows of a K/V head's group in one tile, keys split over a cluster of CTAs; what does
                              // not have that form runs as kind 1
+  kAttnDuo = 7,              // two 128-row tiles, two softmax threads per row, one CTA per SM that walks through the work
+                             // items (5 was kind 1 in that form)
 };
 
 // KIND, D, BLOCK_N, STAGES are compile-time tuning keys (BLOCK_N: KV tile of the single-role kernel, 128
@@ -61,8 +61,9 @@ inline void flash_attn_sm100(const operand_t* q, const operand_t* k, const opera
     rc = sm100::launch_attn_fwd_alt<D, STAGES, 1>(q, k, v, o, shp, st, ex, causal, scale, stream);
   } else if constexpr (KIND == kAttnOneTile) {
     rc = sm100::launch_attn_fwd_one<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
-  } else if constexpr (KIND == kAttnPersistent) {
-    rc = sm100::launch_attn_fwd_pers<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
+  } else if constexpr (KIND == kAttnDuo) {
+    static_assert(BLOCK_N == 128, "written for 128-key tiles");
+    rc = sm100::launch_attn_fwd_duo<D, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
   } else if constexpr (KIND == kAttnFewQueries) {
     if (sm100::split_applies(shp, ex, causal)) {
       rc = sm100::launch_attn_fwd_split<D>(q, k, v, o, shp, st, ex, scale, stream);

@@ -1,0 +1,601 @@
+#pragma once
+// Attention forward for sm_100a with two softmax threads per query row, as a persistent grid.
+//
+// One CTA of 20 warps per SM walks through the work items blockIdx.x, blockIdx.x + gridDim.x, ...; an item is two
+// 128-row query tiles of one (batch, head) slice against all of their KV tiles.
+//   warps 0-15  softmax: query tile (warp >> 2) & 1, keys 64 * (warp >> 3) .. + 63 of every step; warps w and w + 8 hold
+//               the same 32 rows (a warp reaches the 32 tensor-memory lanes of warp & 3 only), thread = row
+//   warp 16     MMA issue for both tiles (warp-uniform code, one elected lane issues)
+//   warp 17     TMA producer (Q tiles, K_j, V_j through a ring of STAGES buffers)
+//   warp 18     TMA stores of finished tiles
+//   warp 19     idle (fills the warpgroup for setmaxnreg)
+//
+// What bounds the kernel is the chain S(j) -> softmax -> P.V(j) -> S(j+1) of each query tile (P overwrites its S, tensor
+// memory has no room for another buffer).  With one thread per row (fwd_ws_sm100.cuh) a tile's softmax is one in-order
+// warp per scheduler: 2100 cycles per step, half of them latency, and 3250 for the chain.  Here each scheduler has two
+// warps per tile, each with half of the exponentials, which cover each other's latencies.  Per step the halves of a row
+// only have to agree on the exponent offset: one OR-reducing barrier of the two warps asks whether any row's maximum
+// outgrew its offset by 2^8 (the lazy-rescale rule), and only then are maxima exchanged and O rescaled, by the softmax
+// warps themselves (S(j) complete implies P.V(j-1) complete: the commit covers it).  There is no correction group.
+//
+//   * P of a half sits in the first 32 columns of that half's 64 score columns, so neither half overwrites scores the
+//     other still needs; the first 32 keys are handed over while the second 32 are fetched from tensor memory again
+//     (keeping them costs registers and lets the compiler move their exponentials in front of the hand-over: 3-5 %).
+//   * Between items (as a CTA's exit and the next one's set-up cost 6-8 us): barriers, tensor memory and the ring live on,
+//     the next item's Q, K and first scores come behind the current item's last steps, accumulators are handed back as
+//     soon as they are in registers, and a warp of its own stores finished tiles from one staging tile that both query
+//     tiles use in turn, which leaves room for four ring slots at head dim 128.
+//   * Values a step does not need are worked out again per item instead of kept: 104 registers hold a half row and its
+//     P without spills (10 % against the first version, which spilled 100 bytes).
+//
+// Measured against the one-thread kernel, both at the clock the board keeps under load (us, same run):
+// 4 x 32 x 4096 x 128 1038 : 1127, causal 561 : 693, 1 x 32 x 16384 causal 2034 : 2211, 2 x 16 x 2048 72 : 77,
+// 16 x 16 x 1024 x 64 103 : 120 (the one-thread kernel's persistent form, which this kernel replaces),
+// 16 x 16 x 1024 x 128 causal 95 : 121, 8 x 16 x 4096 x 64 713 : 835.  3400 cycles per 128 keys of two tiles, tensor pipe
+// active 60 % of a full SM's time, issue slots 43 %.  Tried and left out: 12 or 25 % of the exponentials as a degree-5
+// polynomial on the FMA pipe (-8 %: it lengthens the chain, the special-function unit is not what limits), polling instead
+// of suspending waits in the MMA warp or the softmax warps (level), 6 or 8 ring slots at head dim 64 (level).
+//
+// Every barrier wait is bounded (see sm100_ptx.cuh), and what a warp does next never depends on whether a wait ran out, so
+// the named barriers always meet: a protocol error ends as a status word and a wrong answer, never as a hung GPU.
+
+#include "host_sm100.cuh"
+#include "sm100_ptx.cuh"
+#include "softmax_tile_sm100.cuh"
+
+namespace fray {
+namespace sm100 {
+
+template <int D, int STAGES>
+struct DuoCfg {
+  static_assert(D == 64 || D == 128, "head dim must be 64 or 128");
+  static_assert(STAGES >= 3 && STAGES <= 8, "3..8 K/V buffers");
+  static constexpr int BM = 128, BN = 128;     // rows per query tile, keys per step
+  static constexpr int kThreads = 640;
+  // A half hands its 64 keys to the MMA warp in two chunks of 32, so that half of P.V runs while the second chunk is
+  // still in its exponentials (chunks of 48 + 16 keys: level to 2 % slower).
+  static constexpr int kPChunks = 2;
+  static constexpr int kPanels = D / 64;       // 64-element (128-byte) column panels
+  static constexpr int kQPanelBytes = BM * 128;
+  static constexpr int kQTileBytes = kPanels * kQPanelBytes;
+  static constexpr int kKVPanelBytes = BN * 128;
+  static constexpr int kKVTileBytes = kPanels * kKVPanelBytes;
+  static constexpr int kOffQ = 0;
+  static constexpr int kOffKV = 2 * kQTileBytes;
+  static constexpr int kOffStage = kOffKV + STAGES * kKVTileBytes;  // O staging tile behind the ring, for both query tiles
+  static constexpr int kOffBars = kOffStage + kQTileBytes;
+  static constexpr int kNumBars = 2 * 2 + 2 * STAGES + 2 * 3 + 2 * kPChunks + 2;
+  static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // [2 tiles][2 halves][128]
+  static constexpr int kUsedBytes = kOffStats + 4 * 128 * 4;
+  // slack to bring the dynamic segment to a 1024-byte boundary (its base is one already; the kernel checks)
+  static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
+  static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
+  static constexpr int kTmemCols = 512;
+  static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 384;
+  // Register budgets after setmaxnreg: per scheduler four softmax warps and one other, 4 x 104 + 64 = 5 x 96.
+  static constexpr int kRegsLaunch = 96, kRegsSoftmax = 104, kRegsOther = 64;
+  static constexpr int kRegsTotal = 512 * kRegsSoftmax + 128 * kRegsOther;
+  static_assert(kRegsTotal <= kThreads * kRegsLaunch, "register budgets exceed the CTA's allocation");
+};
+
+// Meets the barrier and returns whether any of its threads passed `p`.
+__device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %3, 0;\n"
+      "barrier.cta.red.or.aligned.pred q, %1, %2, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(id), "r"(threads), "r"(static_cast<uint32_t>(p))
+      : "memory");
+  return r != 0;
+}
+
+// One step of half a row: 64 scores at t_s, the P chunks of 32 keys overwrite their head.
+// my_max: this thread's slot for the exchange of maxima, the other half's is other_off floats away; pair_bar: the named
+// barrier of the two warps that share the rows; lim (MASK): keys from lim on are past the end or above the diagonal.
+template <bool MASK, class Rescale>
+__device__ __forceinline__ void softmax_half(uint32_t t_s, uint64_t* p_bar, float* my_max, int other_off, int pair_bar,
+                                             Rescale&& rescale_o, int lim, float scale_log2, int lane,
+                                             float& m_ref, float& l_run) {
+  uint32_t sa[32], sb[32];
+  tmem_ld_x32(t_s, sa);
+  tmem_ld_x32(t_s + 32, sb);
+  tmem_wait_ld();
+  if constexpr (MASK) {
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      if (c >= lim) sa[c] = __float_as_uint(-INFINITY);
+      if (c + 32 >= lim) sb[c] = __float_as_uint(-INFINITY);
+    }
+  }
+  float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    mx0 = max3(mx0, __uint_as_float(sa[c + 0]), __uint_as_float(sb[c + 0]));
+    mx1 = max3(mx1, __uint_as_float(sa[c + 1]), __uint_as_float(sb[c + 1]));
+    mx2 = max3(mx2, __uint_as_float(sa[c + 2]), __uint_as_float(sb[c + 2]));
+    mx3 = max3(mx3, __uint_as_float(sa[c + 3]), __uint_as_float(sb[c + 3]));
+  }
+  const float mine = fmaxf(max3(mx0, mx1, mx2), mx3);
+  if (named_barrier_or(pair_bar, 64, (mine - m_ref) * scale_log2 > kRescaleThreshold)) {
+    *my_max = mine;
+    named_barrier_sync(pair_bar, 64);
+    const float m_new = max3(mine, my_max[other_off], m_ref);
+    float alpha = 1.f;
+    if ((m_new - m_ref) * scale_log2 > kRescaleThreshold) {
+      // a row without any offset yet has nothing in O (its first product overwrites it)
+      alpha = m_ref == -INFINITY ? 1.f : ex2_approx((m_ref - m_new) * scale_log2);
+      l_run *= alpha;
+      m_ref = m_new;
+    }
+    if (__any_sync(0xffffffffu, alpha != 1.f)) rescale_o(alpha);
+  }
+  const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref * scale_log2;
+  uint64_t rsp0 = 0ull, rsp1 = 0ull;
+  const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2), neg_m2 = pack_f32x2(neg_m, neg_m);
+  auto hand_over = [&](int q) {
+    tmem_wait_st();
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(p_bar + q);
+  };
+  uint32_t pk[16];
+  exp_32(sa, scale2, neg_m2, rsp0, rsp1, pk);
+  tmem_st_x16(t_s, pk);
+  tmem_ld_x32(t_s + 32, sb);
+  hand_over(0);
+  tmem_wait_ld();
+  if constexpr (MASK) {
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+      if (c + 32 >= lim) sb[c] = __float_as_uint(-INFINITY);
+  }
+  uint32_t pk2[16];
+  exp_32(sb, scale2, neg_m2, rsp0, rsp1, pk2);
+  tmem_st_x16(t_s + 16, pk2);
+  hand_over(1);
+  float r0, r1, r2, r3;
+  unpack_f32x2(rsp0, r0, r1);
+  unpack_f32x2(rsp1, r2, r3);
+  l_run += (r0 + r1) + (r2 + r3);
+}
+
+// One work item: the rows [m0, m0 + 256) of slice (b, h) and the KV tiles each of its two query tiles consumes.
+struct DuoItem {
+  int m0, b, h, n0, n1;
+};
+
+template <int D, int STAGES>
+__global__ void __launch_bounds__(640, 1)
+attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
+                    int num_heads, int num_bh, int seq_len, int causal, float scale_log2, int kv_group, float* lse, int seq_k,
+                    int blk, int n_kv, int n_pairs, int total) {
+  using Cfg = DuoCfg<D, STAGES>;
+  constexpr int BN = Cfg::BN;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t align_off = ((raw_addr + 1023u) & ~1023u) - raw_addr;
+  uint8_t* smem = smem_raw + align_off;
+  uint8_t* q_smem = smem + Cfg::kOffQ;
+  uint8_t* kv_smem = smem + Cfg::kOffKV;
+  uint8_t* stage_smem = smem + Cfg::kOffStage;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
+  uint64_t* q_full = bars;                      // [2]   producer -> MMA
+  uint64_t* q_free = bars + 2;                  // [2]   MMA -> producer  (the item's last S of tile i has read Q_i)
+  uint64_t* kv_full = bars + 4;                 // [STAGES] producer -> MMA
+  uint64_t* kv_empty = kv_full + STAGES;        // [STAGES] MMA -> producer
+  uint64_t* s_full = kv_empty + STAGES;         // [2]   MMA -> softmax i
+  uint64_t* o_full = s_full + 2;                // [2]   MMA -> softmax i (the item's last P.V)
+  uint64_t* o_free = o_full + 2;                // [2]   softmax i -> MMA (the item's O_i is in registers)
+  uint64_t* p_full = o_free + 2;                // [2][kPChunks] softmax i -> MMA
+  uint64_t* stage_full = p_full + 2 * Cfg::kPChunks;  // softmax -> store warp
+  uint64_t* stage_free = stage_full + 1;        // store warp -> softmax
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
+  float* stats = reinterpret_cast<float*>(smem + Cfg::kOffStats);
+
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+
+  if (align_off + Cfg::kUsedBytes > Cfg::kSmemBytes) {  // never seen: the segment's base is 1024-byte aligned
+    if (tid == 0) atomicCAS(&fray_attn_status[0], 0, 0x601);
+    return;
+  }
+
+  const int stride = static_cast<int>(gridDim.x);
+  // Items are numbered in blocks of `blk` slices; inside a block the pairs of all its slices come heaviest first (pair by
+  // pair, slice by slice).  blk = 1 is plain slice order: CTAs that run side by side share a slice's K and V in L2.  A
+  // causal problem of few, unequal items takes blk = all slices (heaviest_first_order has the measurements).  CTA c takes
+  // the positions c, G + c, 2G + c, ...; with a causal mask the direction alternates from round to round, which evens
+  // out most of what is left.
+  auto pos = [&](int k) {
+    const int c = static_cast<int>(blockIdx.x);
+    return k * stride + ((causal && (k & 1)) ? stride - 1 - c : c);  // >= total: the CTA is done; grows with k
+  };
+  auto decode = [&](int idx) {
+    DuoItem it;
+    const int blk_items = blk * n_pairs;
+    const int blk_i = idx / blk_items;
+    const int rem = idx - blk_i * blk_items;
+    const int left = num_bh - blk_i * blk;
+    const int ns = left < blk ? left : blk;
+    const int pr = rem / ns;
+    const int bh = blk_i * blk + (rem - pr * ns);
+    const int pair = causal ? (n_pairs - 1 - pr) : pr;
+    it.m0 = pair * (2 * Cfg::BM);
+    it.b = bh / num_heads;
+    it.h = bh - it.b * num_heads;
+    int n[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row0 = it.m0 + i * Cfg::BM;
+      n[i] = row0 < seq_len ? n_kv : 0;
+      if (causal && n[i] > 0) {
+        const int lim = (row0 + Cfg::BM + BN - 1) / BN;
+        n[i] = lim < n[i] ? lim : n[i];
+      }
+    }
+    it.n0 = n[0];
+    it.n1 = n[1];
+    return it;
+  };
+
+  if (tid == 0) {
+    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(q_full + i, 1);
+      mbar_init(q_free + i, 1);
+      mbar_init(s_full + i, 1);
+      for (int c = 0; c < Cfg::kPChunks; ++c) mbar_init(p_full + i * Cfg::kPChunks + c, 8);
+      mbar_init(o_full + i, 1);
+      mbar_init(o_free + i, 8);
+    }
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(kv_full + s, 1);
+      mbar_init(kv_empty + s, 1);
+    }
+    mbar_init(stage_full, 8);
+    mbar_init(stage_free, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (*abort_flag != 0) return;
+
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < 16) {
+    // =============================================================== softmax
+    set_max_regs_inc<Cfg::kRegsSoftmax>();
+    const int i = (warp >> 2) & 1;  // query tile
+    const int hf = warp >> 3;       // which 64 keys of a step, which D / 2 columns of O
+    const int r = tid & 127;        // row inside the tile
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem_base + (i == 0 ? Cfg::kColS0 : Cfg::kColS1) + hf * 64 + lane_base;
+    const uint32_t t_o = tmem_base + (i == 0 ? Cfg::kColO0 : Cfg::kColO1) + hf * (D / 2) + lane_base;
+    uint64_t* p_bar = p_full + i * Cfg::kPChunks;
+    float* my_stat = stats + (i * 2 + hf) * 128 + r;
+    const int other_off = hf ? -128 : 128;
+    const int pair_bar = 1 + i * 4 + (warp & 3);
+    auto rescale_o = [&](float alpha) {
+#pragma unroll 1
+      for (int c = 0; c < D / 2; c += 16) {
+        uint32_t orr[16];
+        tmem_ld_x16(t_o + c, orr);
+        tmem_wait_ld();
+#pragma unroll
+        for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+        tmem_st_x16(t_o + c, orr);
+      }
+      tmem_wait_st();
+    };
+    // phase parities, toggled: bit 0 s_full, bit 1 o_full, bits 2.. tiles of either index staged before
+    uint32_t phases = 0;
+    for (int k = 0, idx = pos(0); idx < total; idx = pos(++k)) {
+      int n_i, row0;
+      uint32_t my_store;
+      {
+        const DuoItem it = decode(idx);
+        n_i = i ? it.n1 : it.n0;
+        row0 = it.m0 + i * Cfg::BM;
+        my_store = (phases >> 2) + (i && it.n0 > 0);
+        phases += 4u * ((it.n0 > 0) + (it.n1 > 0));
+      }
+      if (n_i == 0) continue;
+      // the first steps see every key of their tile
+      int n_full = seq_k / BN;
+      if (causal) n_full = (row0 + 1) / BN < n_full ? (row0 + 1) / BN : n_full;
+      if (n_full > n_i) n_full = n_i;
+      float m_ref = -INFINITY;
+      float l_run = 0.f;
+      for (int j = 0; j < n_full; ++j) {
+        mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+        tc_fence_after_sync();
+        softmax_half<false>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, 0, scale_log2, lane, m_ref, l_run);
+        phases ^= 1u;
+      }
+      {
+        const int row = row0 + r;
+        int lim = (causal && row + 1 < seq_k ? row + 1 : seq_k) - hf * 64 - n_full * BN;  // keys the row may see from here
+        for (int j = n_full; j < n_i; ++j, lim -= BN) {
+          mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+          tc_fence_after_sync();
+          softmax_half<true>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, lim, scale_log2, lane, m_ref, l_run);
+          phases ^= 1u;
+        }
+      }
+      *my_stat = l_run;
+      named_barrier_sync(pair_bar, 64);
+      l_run += my_stat[other_off];
+      named_barrier_sync(pair_bar, 64);  // the slots take the next item's maxima
+      if (my_store > 0) mbar_wait(stage_free, (my_store - 1) & 1, abort_flag, 0x321 + i, idx);
+      mbar_wait(o_full + i, (phases >> 1) & 1, abort_flag, 0x331 + i, idx);
+      phases ^= 2u;
+      tc_fence_after_sync();
+      const float inv_l = l_run > 0.f ? 1.f / l_run : 1.f;
+#pragma unroll
+      for (int c = 0; c < D / 2; c += 32) {
+        uint32_t orr[32];
+        tmem_ld_x32(t_o + c, orr);
+        tmem_wait_ld();
+        if (c + 32 == D / 2) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(o_free + i);
+        }
+        const int col = hf * (D / 2) + c;  // first column of these 32
+        uint8_t* panel_row = stage_smem + (col >> 6) * Cfg::kQPanelBytes + r * 128;
+#pragma unroll
+        for (int x = 0; x < 32; x += 8) {
+          uint4 v4;
+          v4.x = pack_half2(__uint_as_float(orr[x + 0]) * inv_l, __uint_as_float(orr[x + 1]) * inv_l);
+          v4.y = pack_half2(__uint_as_float(orr[x + 2]) * inv_l, __uint_as_float(orr[x + 3]) * inv_l);
+          v4.z = pack_half2(__uint_as_float(orr[x + 4]) * inv_l, __uint_as_float(orr[x + 5]) * inv_l);
+          v4.w = pack_half2(__uint_as_float(orr[x + 6]) * inv_l, __uint_as_float(orr[x + 7]) * inv_l);
+          const int chunk = ((col & 63) + x) >> 3;  // 16-byte chunk inside the 128-byte row
+          *reinterpret_cast<uint4*>(panel_row + ((chunk ^ (r & 7)) << 4)) = v4;
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(stage_full);
+      if (lse != nullptr && hf == 0 && row0 + r < seq_len) {
+        int again = idx;
+        asm volatile("" : "+r"(again));  // worked out again here instead of kept through the steps
+        const DuoItem it = decode(again);
+        lse[(static_cast<size_t>(it.b) * num_heads + it.h) * seq_len + row0 + r] =
+            l_run > 0.f ? (m_ref * scale_log2 + log2f(l_run)) * 0.69314718055994531f : -INFINITY;
+      }
+    }
+  } else {
+    set_max_regs_dec<Cfg::kRegsOther>();
+    if (warp == 18 && lane == 0) {
+      // ============================================================= stores of finished tiles
+      uint32_t stores = 0;
+      for (int k = 0, idx = pos(0); idx < total; idx = pos(++k)) {
+        const DuoItem it = decode(idx);
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+          if ((i ? it.n1 : it.n0) == 0) continue;
+          mbar_wait(stage_full, stores & 1, abort_flag, 0x341 + i, idx);
+          if (*abort_flag != 0) break;
+#pragma unroll
+          for (int p = 0; p < Cfg::kPanels; ++p)
+            tma_store_4d(&tm_o, stage_smem + p * Cfg::kQPanelBytes, p * 64, it.m0 + i * Cfg::BM, it.h, it.b);
+          tma_store_commit();
+          tma_store_wait_read();
+          mbar_arrive(stage_free);
+          ++stores;
+        }
+      }
+    } else if (warp == 17 && lane == 0) {
+      // ============================================================= TMA producer
+      uint32_t t_run = 0;               // K/V tiles loaded so far: ring slot and phase
+      uint32_t q_cnt0 = 0, q_cnt1 = 0;  // items whose Q_0 / Q_1 this CTA has loaded
+      for (int k = 0, idx = pos(0); idx < total; idx = pos(++k)) {
+        const DuoItem it = decode(idx);
+        const int h_kv = it.h / kv_group;
+        const int n_max = it.n0 > it.n1 ? it.n0 : it.n1;
+        auto load_q = [&](int i) __attribute__((always_inline)) {
+          if ((i ? it.n1 : it.n0) > 0) {
+            const uint32_t cnt = i ? q_cnt1 : q_cnt0;
+            if (cnt > 0) mbar_wait(q_free + i, (cnt - 1) & 1, abort_flag, 0x402 + i, idx);
+            mbar_expect_tx(q_full + i, Cfg::kQTileBytes);
+#pragma unroll
+            for (int p = 0; p < Cfg::kPanels; ++p)
+              tma_load_4d(q_smem + i * Cfg::kQTileBytes + p * Cfg::kQPanelBytes, &tm_q, q_full + i, p * 64,
+                          it.m0 + i * Cfg::BM, it.h, it.b);
+            if (i) ++q_cnt1; else ++q_cnt0;
+          }
+        };
+        load_q(0);
+        for (int t = 0; t < 2 * n_max; ++t) {
+          const int slot = t_run % STAGES;
+          const uint32_t ph = (t_run / STAGES) & 1;
+          mbar_wait(kv_empty + slot, ph ^ 1, abort_flag, 0x401, t);
+          if (*abort_flag != 0) break;
+          mbar_expect_tx(kv_full + slot, Cfg::kKVTileBytes);
+          const CUtensorMap* tm = (t & 1) ? &tm_v : &tm_k;
+#pragma unroll
+          for (int p = 0; p < Cfg::kPanels; ++p)
+            tma_load_4d(kv_smem + slot * Cfg::kKVTileBytes + p * Cfg::kKVPanelBytes, tm, kv_full + slot, p * 64,
+                        (t >> 1) * BN, h_kv, it.b);
+          ++t_run;
+          if (t == 0) load_q(1);
+        }
+        if (*abort_flag != 0) break;
+      }
+    } else if (warp == 16) {
+      // ============================================================= MMA issue (whole warp, one elected lane issues)
+      constexpr uint64_t kDescK = smem_desc_sw128(16, 1024);
+      constexpr uint64_t kDescV = smem_desc_sw128(Cfg::kKVPanelBytes, 1024);
+      constexpr uint32_t kIdescQK = idesc_f16_f32(Cfg::BM, BN, false, false);
+      constexpr uint32_t kIdescPV = idesc_f16_f32(Cfg::BM, D, false, true);
+      const uint32_t q_addr = smem_u32(q_smem);
+      const uint32_t kv_addr = smem_u32(kv_smem);
+      // phase parities of tile 0 / 1: bits 0, 1 p_full; bits 2, 3 q_full; bits 4, 5 o_free (parity 1 at first: the
+      // accumulators are free)
+      uint32_t phases = 0x30;
+
+      auto wait_kv = [&](uint32_t t_abs, int j) __attribute__((always_inline)) {
+        mbar_wait(kv_full + t_abs % STAGES, (t_abs / STAGES) & 1, abort_flag, 0x501, j);
+      };
+      // S_i(j) = Q_i . K_j^T of item `it` (ring index t_abs)
+      auto issue_qk = [&](int i, const DuoItem& it, int j, uint32_t t_abs) __attribute__((always_inline)) {
+        const int slot = t_abs % STAGES;
+        tc_fence_after_sync();
+        constexpr uint32_t kDescHi = static_cast<uint32_t>(kDescK >> 32);
+        constexpr uint32_t kDescLo = static_cast<uint32_t>(kDescK);
+        uint32_t q_lo = kDescLo | (((q_addr + i * Cfg::kQTileBytes) & 0x3FFFF) >> 4);
+        uint32_t k_lo = kDescLo | (((kv_addr + slot * Cfg::kKVTileBytes) & 0x3FFFF) >> 4);
+        uint32_t t_s = tmem_base + (i == 0 ? Cfg::kColS0 : Cfg::kColS1);
+        asm volatile("" : "+r"(q_lo), "+r"(k_lo), "+r"(t_s));  // keeps the unrolled addresses out of registers across steps
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t qoff = ((kk >> 2) * Cfg::kQPanelBytes + (kk & 3) * 32) >> 4;
+          const uint32_t koff = ((kk >> 2) * Cfg::kKVPanelBytes + (kk & 3) * 32) >> 4;
+          mma_ss_elect_lohi(t_s, q_lo + qoff, kDescHi, k_lo + koff, kDescHi, kIdescQK, kk > 0);
+        }
+        mma_commit_elect(s_full + i);
+        if ((i == 1) || !(j < it.n1)) mma_commit_elect(kv_empty + slot);
+        if (j + 1 == (i ? it.n1 : it.n0)) mma_commit_elect(q_free + i);
+      };
+      auto issue_pv = [&](int i, const DuoItem& it, int j, uint32_t t_abs) __attribute__((always_inline)) {
+        const int slot = t_abs % STAGES;
+        const bool last = j + 1 == (i ? it.n1 : it.n0);
+        wait_kv(t_abs, j);
+        if (j == 0) {
+          // the first product of an item overwrites O: the previous item's epilogue must have read it
+          mbar_wait(o_free + i, (phases >> (4 + i)) & 1, abort_flag, 0x507 + i, j);
+          phases ^= 0x10u << i;
+        }
+        if (!last) wait_kv(t_abs + 1, j);  // the next K tile: ahead of P, off the path to the next scores
+        constexpr uint32_t kDescVHi = static_cast<uint32_t>(kDescV >> 32);
+        uint32_t v_lo = static_cast<uint32_t>(kDescV) | (((kv_addr + slot * Cfg::kKVTileBytes) & 0x3FFFF) >> 4);
+        uint32_t t_p = tmem_base + (i == 0 ? Cfg::kColS0 : Cfg::kColS1);
+        uint32_t t_o = tmem_base + (i == 0 ? Cfg::kColO0 : Cfg::kColO1);
+        asm volatile("" : "+r"(v_lo), "+r"(t_p), "+r"(t_o));
+        const uint32_t ph = (phases >> i) & 1;
+#pragma unroll
+        for (int q = 0; q < Cfg::kPChunks; ++q) {
+          mbar_wait(p_full + i * Cfg::kPChunks + q, ph, abort_flag, 0x503 + i, j);
+          tc_fence_after_sync();
+#pragma unroll
+          for (int s2 = 0; s2 < 4; ++s2) {
+            // 16 keys per MMA: the chunk's 32 keys of either half; a half's P sits in columns [0,32) / [64,96)
+            const int kk = (s2 >> 1) * 4 + q * 2 + (s2 & 1);
+            mma_ts_elect_lohi(t_o, t_p + (kk >> 2) * 64 + (kk & 3) * 8, v_lo + ((kk * 2048) >> 4), kDescVHi, kIdescPV,
+                              (j > 0 || q > 0 || s2 > 0));
+          }
+        }
+        phases ^= 1u << i;
+        if (last) mma_commit_elect(o_full + i);
+        if ((i == 1) || !(j < it.n1)) mma_commit_elect(kv_empty + slot);
+      };
+      auto first_qk = [&](int i, const DuoItem& it, uint32_t t_abs) __attribute__((always_inline)) {
+        mbar_wait(q_full + i, (phases >> (2 + i)) & 1, abort_flag, 0x511 + i);
+        phases ^= 4u << i;
+        wait_kv(t_abs, 0);
+        issue_qk(i, it, 0, t_abs);
+      };
+
+      int k = 0;
+      const int idx = pos(0);
+      if (idx < total) {
+        DuoItem cur = decode(idx);
+        uint32_t t_base = 0;  // ring index of the current item's K_0
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i)
+          if ((i ? cur.n1 : cur.n0) > 0) first_qk(i, cur, t_base);
+        while (true) {
+          const int idx_next = pos(k + 1);
+          const bool has_next = idx_next < total;
+          DuoItem nxt = cur;
+          nxt.n0 = 0;
+          nxt.n1 = 0;
+          if (has_next) nxt = decode(idx_next);
+          const int n_max = cur.n0 > cur.n1 ? cur.n0 : cur.n1;
+          const uint32_t t_next = t_base + 2 * n_max;
+          for (int j = 0; j < n_max; ++j) {
+#pragma unroll 1
+            for (int i = 0; i < 2; ++i) {
+              const int n_i = i ? cur.n1 : cur.n0;
+              if (j < n_i) {
+                issue_pv(i, cur, j, t_base + 2 * j + 1);
+                if (j + 1 < n_i) {
+                  issue_qk(i, cur, j + 1, t_base + 2 * (j + 1));
+                } else if ((i ? nxt.n1 : nxt.n0) > 0 && (i == 1 || cur.n0 == cur.n1)) {
+                  first_qk(i, nxt, t_next);  // the next item's first scores, right behind this item's last P.V
+                }
+              }
+            }
+            // A tile 0 that ends a step before tile 1: its next first scores go behind tile 1's product of this
+            // step, which hands back the ring slot the next item's K_0 needs.
+            if (cur.n0 != cur.n1 && j + 1 == cur.n0 && nxt.n0 > 0) first_qk(0, nxt, t_next);
+          }
+          // a tile that had nothing to do in this item (past the last query) but has in the next
+#pragma unroll 1
+          for (int i = 0; i < 2; ++i)
+            if ((i ? cur.n1 : cur.n0) == 0 && (i ? nxt.n1 : nxt.n0) > 0) first_qk(i, nxt, t_next);
+          if (!has_next) break;
+          cur = nxt;
+          t_base = t_next;
+          ++k;
+        }
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+}
+
+// Host launcher for the kernel with two softmax threads per row. Returns an AttnReturnCode.
+template <int D, int STAGES>
+inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const operand_t* v, operand_t* o, const AttnShape& shp,
+                               const AttnStrides (&st)[4], const AttnExtras& ex, bool causal, float scale,
+                               cudaStream_t stream) {
+  using Cfg = DuoCfg<D, STAGES>;
+  const AttnShape shp_kv{shp.B, shp.H / ex.kv_group, ex.seq_k, shp.D};
+  CUtensorMap tm_q, tm_k, tm_v, tm_o;
+  int rc = cached_attn_tensor_map(&tm_q, q, shp, st[0], Cfg::BM);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_k, k, shp_kv, st[1], Cfg::BN);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_v, v, shp_kv, st[2], Cfg::BN);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_o, o, shp, st[3], Cfg::BM);
+  if (rc != kAttnOk) return rc;
+
+  auto kernel = attn_fwd_duo_kernel<D, STAGES>;
+  rc = ensure_dynamic_smem<Cfg>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
+  if (rc != kAttnOk) return rc;
+  const int sms = device_sm_count();
+  if (sms <= 0) return kAttnLaunchFailed;
+  const int n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
+  const int items = n_pairs * shp.B * shp.H;
+  const int grid = items < sms ? items : sms;
+  // item order (see the kernel): heaviest first over all slices or slice by slice
+  const int blk = heaviest_first_order(causal, shp, shp_kv) ? shp.B * shp.H : 1;
+  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0,
+                                                           scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k, blk,
+                                                           (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
+  if (cudaGetLastError() != cudaSuccess) return kAttnLaunchFailed;
+  return kAttnOk;
+}
+
+}  // namespace sm100
+}  // namespace fray
