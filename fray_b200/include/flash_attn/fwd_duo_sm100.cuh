@@ -247,7 +247,6 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
     for (int i = 0; i < 2; ++i) {
       mbar_init(q_full + i, 1);
       mbar_init(q_free + i, 1);
@@ -264,17 +263,22 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     mbar_init(stage_free, 1);
     fence_barrier_init();
   }
-  __syncthreads();
-  if (*abort_flag != 0) return;
-
+  __syncwarp();
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
+  if (*abort_flag != 0) {  // an earlier launch left the device status raised
+    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    return;
+  }
 
   if (warp < 16) {
     // =============================================================== softmax
@@ -590,11 +594,9 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
   const int grid = items < sms ? items : sms;
   // item order (see the kernel): heaviest first over all slices or slice by slice
   const int blk = heaviest_first_order(causal, shp, shp_kv) ? shp.B * shp.H : 1;
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0,
-                                                           scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k, blk,
-                                                           (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
-  if (cudaGetLastError() != cudaSuccess) return kAttnLaunchFailed;
-  return kAttnOk;
+  return launch_overlapped(kernel, dim3(grid), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, tm_o, shp.H,
+                           shp.B * shp.H, shp.S, causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse,
+                           ex.seq_k, blk, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
 }
 
 }  // namespace sm100

@@ -106,7 +106,6 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
     mbar_init(q_full, 1);
     mbar_init(s_full, 1);
     mbar_init(o_full, 1);
@@ -118,19 +117,24 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     fence_barrier_init();
     prefetch_tensormap(&tm_o);
   }
-  __syncthreads();
-  if (*abort_flag != 0) return;  // an earlier launch left the device status raised
-
+  __syncwarp();
   if (warp == 0) {
     // two CTAs of an SM allocate 256 columns each; the allocation waits inside the instruction until the
     // columns are there, which they are as soon as an earlier CTA of the SM has freed its own
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
+  if (*abort_flag != 0) {  // an earlier launch left the device status raised
+    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    return;
+  }
 
   if (warp < 4) {
     // =============================================================== softmax group
@@ -291,11 +295,9 @@ inline int launch_attn_fwd_one(const operand_t* q, const operand_t* k, const ope
   const int heaviest_first = heaviest_first_order(causal, shp, shp_kv) ? 1 : 0;
   const unsigned n_x = (shp.S + Cfg::BM - 1) / (Cfg::BM), n_bh = shp.B * shp.H;
   dim3 grid(heaviest_first ? n_bh : n_x, heaviest_first ? n_x : n_bh);
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_o, shp.H, shp.S, causal ? 1 : 0,
-                                                           scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k,
-                                                           heaviest_first);
-  if (cudaGetLastError() != cudaSuccess) return kAttnLaunchFailed;
-  return kAttnOk;
+  return launch_overlapped(kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, tm_o, shp.H, shp.S,
+                           causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k,
+                           heaviest_first);
 }
 
 }  // namespace sm100

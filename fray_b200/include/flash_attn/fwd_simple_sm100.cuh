@@ -66,7 +66,6 @@ attn_fwd_simple_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const int h_kv = h / kv_group;  // K/V head of this query head (one division per CTA, not per copy)
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
     mbar_init(bar_q, 1);
     mbar_init(bar_k, 1);
     mbar_init(bar_v, 1);
@@ -77,17 +76,22 @@ attn_fwd_simple_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     prefetch_tensormap(&tm_k);
     prefetch_tensormap(&tm_v);
   }
-  __syncthreads();
-  if (*abort_flag != 0) return;  // an earlier launch left the device status raised
-
+  __syncwarp();
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
+  if (*abort_flag != 0) {  // an earlier launch left the device status raised
+    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    return;
+  }
   const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
   const uint32_t t_s = tmem_base + Cfg::kColS;
   const uint32_t t_o = tmem_base + Cfg::kColO;
@@ -255,10 +259,9 @@ inline int launch_attn_fwd_simple(const operand_t* q, const operand_t* k, const 
   rc = ensure_dynamic_smem<Cfg>(kernel, Cfg::kSmemBytes);
   if (rc != kAttnOk) return rc;
   dim3 grid((shp.S + Cfg::BM - 1) / Cfg::BM, shp.B * shp.H);
-  kernel<<<grid, 128, Cfg::kSmemBytes, stream>>>(tm_q, tm_k, tm_v, o, st[3].b, st[3].h, st[3].s, shp.H, shp.S,
-                                                 causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k);
-  if (cudaGetLastError() != cudaSuccess) return kAttnLaunchFailed;
-  return kAttnOk;
+  return launch_overlapped(kernel, grid, 128, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, o, st[3].b, st[3].h, st[3].s,
+                           shp.H, shp.S, causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse,
+                           ex.seq_k);
 }
 
 }  // namespace sm100

@@ -104,7 +104,6 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int t_last = static_cast<int>(static_cast<long long>(n_kv) * (split + 1) / splits);
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
     mbar_init(q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(kv_full + s, 1);
@@ -122,9 +121,12 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   // An earlier launch left the device status raised: compute nothing, but meet the cluster's barriers.
   const bool dead = *abort_flag != 0;
@@ -414,12 +416,14 @@ inline int launch_attn_fwd_split_copies(const operand_t* q, const operand_t* k, 
   cfg.blockDim = dim3(Cfg::kThreads);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   auto clusters_of = [&](int c) {
     cfg.gridDim = dim3(c, units);
     attr[0].val.clusterDim.x = c;

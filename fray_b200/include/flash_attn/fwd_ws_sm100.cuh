@@ -144,7 +144,6 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (tid == 0) {
     FRAY_TRACE(6, 0, 0);  // CTA entry
     FRAY_TRACE_NS(6, 0, 10);
-    *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
     for (int i = 0; i < 2; ++i) {
       mbar_init(q_full + i, 1);
       mbar_init(s_full + i, 1);
@@ -160,17 +159,22 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     fence_barrier_init();
     prefetch_tensormap(&tm_o);
   }
-  __syncthreads();
-  if (*abort_flag != 0) return;  // an earlier launch left the device status raised
-
+  __syncwarp();
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();
+  if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
+  if (*abort_flag != 0) {  // an earlier launch left the device status raised
+    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    return;
+  }
   if (tid == 0) FRAY_TRACE(6, 0, 1);  // set-up done
 
   // (rotating the role assignment over the warp index was measured to make no difference)
@@ -401,11 +405,9 @@ inline int launch_attn_fwd_ws(const operand_t* q, const operand_t* k, const oper
   const int group_slices = heaviest_first_group(causal, shp, shp_kv);
   const unsigned n_x = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM), n_bh = shp.B * shp.H;
   dim3 grid = group_slices > 0 ? dim3(group_slices, n_x, (n_bh + group_slices - 1) / group_slices) : dim3(n_x, n_bh);
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_o, shp.H, shp.S, causal ? 1 : 0,
-                                                           scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k,
-                                                           group_slices, static_cast<int>(n_bh));
-  if (cudaGetLastError() != cudaSuccess) return kAttnLaunchFailed;
-  return kAttnOk;
+  return launch_overlapped(kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, tm_o, shp.H, shp.S,
+                           causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse, ex.seq_k,
+                           group_slices, static_cast<int>(n_bh));
 }
 
 }  // namespace sm100

@@ -176,6 +176,29 @@ inline int ensure_dynamic_smem(Kernel kernel, int bytes, int threads = 0, int re
   return kAttnOk;
 }
 
+// Launches a kernel whose CTAs may be set up (barriers, tensor memory) while the stream's previous kernel drains; the
+// kernel itself waits for that one's end before it touches global memory (grid_dependency_wait).  Per call, back to back
+// on one stream: 6 x 12 x 333 x 64 causal 12.3 -> 10.9 us, 2 x 16 x 2048 x 128 78.8 -> 77.0, 8 x 8 x 8192 decode
+// 52.2 -> 51.3; nothing from 100 us on.
+template <class... Params, class... Args>
+inline int launch_overlapped(void (*kernel)(Params...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return kAttnLaunchFailed;
+  }
+  return kAttnOk;
+}
+
 // Order in which the query tiles of a causal problem start: slice by slice (CTAs side by side share a slice's
 // K and V in L2), or the heaviest tiles of ALL (batch, head) slices first, which lets the hardware's
 // first-come scheduling even out the tiles' unequal lengths.  Measured on 4096- and 16384-row causal problems,

@@ -139,6 +139,14 @@ __device__ __forceinline__ void mbar_wait_spin(uint64_t* bar, uint32_t parity, v
   }
 }
 
+// ---------------------------------------------------------------- overlap with the stream's neighbours
+// A kernel launched with launch_overlapped may start while the kernel before it in the stream still runs: everything it
+// reads or writes in global memory comes after this wait (the earlier kernel has ended and its writes are visible).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start its CTAs, once every CTA of this one has come here, where this one's leave
+// room.  Only after the CTA's tensor memory is allocated: a waiting successor may hold columns itself.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- CTA pairs (clusters of two)
 // Rank of this CTA inside its cluster (0 for a kernel launched without clusters).
 __device__ __forceinline__ uint32_t cluster_ctarank() {
