@@ -77,4 +77,21 @@ inline void flash_attn_sm100(const operand_t* q, const operand_t* k, const opera
   }
 }
 
+// The arguments of flash_attn_sm100 that stay the same from call to call of one tensor layout.
+struct AttnLayout {
+  int batch_size, num_heads, seq_len;
+  int q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh, o_ss;
+  int num_kv_heads, seq_len_kv, causal;
+  float scale;
+};
+
+template <int KIND, int D, int BLOCK_N, int STAGES>
+inline void flash_attn_layout(void* q, void* k, void* v, void* o, void* lse, void* stream, const AttnLayout& l, int& rc) {
+  flash_attn_sm100<KIND, D, BLOCK_N, STAGES>(
+      static_cast<const operand_t*>(q), static_cast<const operand_t*>(k), static_cast<const operand_t*>(v),
+      static_cast<operand_t*>(o), l.batch_size, l.num_heads, l.seq_len, l.q_sb, l.q_sh, l.q_ss, l.k_sb, l.k_sh, l.k_ss,
+      l.v_sb, l.v_sh, l.v_ss, l.o_sb, l.o_sh, l.o_ss, l.num_kv_heads, l.seq_len_kv, static_cast<float*>(lse), l.causal != 0,
+      l.scale, static_cast<cudaStream_t>(stream), rc);
+}
+
 }  // namespace fray
