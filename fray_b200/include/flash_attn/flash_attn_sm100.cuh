@@ -26,7 +26,8 @@ enum AttnKernelKind : int {
   kAttnFewQueries = 6,       // all rows of a K/V head's group in one tile, keys split over a cluster of CTAs; what does
                              // not have that form runs as kind 1
   kAttnDuo = 7,              // two 128-row tiles, two softmax threads per row, one CTA per SM that walks through the work
-                             // items (5 was kind 1 in that form)
+                             // items
+  kAttnPersistent = 5,       // kind 1 in that form, until kind 7 was faster in all of it: the number now means kind 7
 };
 
 // KIND, D, BLOCK_N, STAGES are compile-time tuning keys (BLOCK_N: KV tile of the single-role kernel, 128
@@ -61,7 +62,7 @@ inline void flash_attn_sm100(const operand_t* q, const operand_t* k, const opera
     rc = sm100::launch_attn_fwd_alt<D, STAGES, 1>(q, k, v, o, shp, st, ex, causal, scale, stream);
   } else if constexpr (KIND == kAttnOneTile) {
     rc = sm100::launch_attn_fwd_one<D, BLOCK_N, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
-  } else if constexpr (KIND == kAttnDuo) {
+  } else if constexpr (KIND == kAttnDuo || KIND == kAttnPersistent) {
     static_assert(BLOCK_N == 128, "written for 128-key tiles");
     rc = sm100::launch_attn_fwd_duo<D, STAGES>(q, k, v, o, shp, st, ex, causal, scale, stream);
   } else if constexpr (KIND == kAttnFewQueries) {

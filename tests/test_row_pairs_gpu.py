@@ -1,0 +1,42 @@
+"""The kernel with two softmax threads per row, forced: more work items than SMs, ragged ends, moving offsets."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# items = slices * ceil(Sq / 256): fewer than SMs, more than one and more than two rounds; a second tile that is empty
+# (Sq % 256 <= 128), one that holds a single row, one KV tile only, keys ending inside either half of a step
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,causal", [
+    (1, 3, 3, 129, 129, True), (3, 60, 60, 300, 300, True), (3, 60, 20, 257, 190, False), (2, 100, 100, 100, 128, False),
+    (1, 160, 160, 640, 640, True), (2, 90, 9, 513, 1000, False), (1, 2, 1, 2000, 70, True), (1, 5, 5, 4100, 4100, True)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("gain", [1.0, 6.0])
+def test_row_pairs(B, H, Hkv, Sq, Sk, causal, D, gain, monkeypatch):
+    import importlib
+    op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
+    monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
+    point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
+    monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    g = torch.Generator(device="cuda").manual_seed(81)
+    q = (gain * torch.randn(B, H, Sq, D, generator=g, device="cuda")).half()  # gain 6: offsets move during a row
+    k, v = (torch.randn(B, Hkv, Sk, D, generator=g, device="cuda").half() for _ in range(2))
+    guard = torch.full((B, H, Sq + 1, D), 7.0, dtype=torch.half, device="cuda")
+    lse = torch.zeros(B, H, Sq, device="cuda")
+    op.flash_attn_cute(q, k, v, guard[:, :, :Sq], causal=causal, lse=lse)
+    torch.cuda.synchronize()
+    assert op.flash_attn_status()[0] == 0
+    assert (guard[:, :, Sq:] == 7.0).all()
+    mask = torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril() if causal else None
+    for b in range(B):  # a batch at a time bounds the 64-bit scores
+        ke, ve = (t[b].repeat_interleave(H // Hkv, 0).double() for t in (k, v))
+        s = q[b].double() @ ke.transpose(-1, -2) / math.sqrt(D)
+        if causal:
+            s.masked_fill_(~mask, float("-inf"))
+        # fp16 rounds to within 2^-11 of a value: every P by that much, which moves a convex sum of |v| <= 6 by at most
+        # 6 * 2^-11, and the output once more
+        assert (guard[b, :, :Sq].double() - torch.softmax(s, -1) @ ve).abs().max().item() <= 2 * 6 * 2.0 ** -11
+        assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() <= 2e-4
+        del s
