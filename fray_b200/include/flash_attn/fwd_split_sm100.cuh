@@ -379,6 +379,7 @@ inline int split_count(int units, int n_kv, const int (&active)[SplitCfg<128>::k
   int best = 1;
   long long best_cost = -1;
   for (int c = 1; c <= SplitCfg<128>::kMaxSplits && c <= n_kv; ++c) {
+    if (active[c] <= 0) continue;
     const long long rounds = (static_cast<long long>(units) + active[c] - 1) / active[c];
     const long long cost = rounds * ((n_kv + c - 1) / c + 3);
     if (best_cost < 0 || cost < best_cost) {
@@ -439,11 +440,12 @@ inline int launch_attn_fwd_split_copies(const operand_t* q, const operand_t* k, 
   if (dev != active_dev) {
     for (int c = 1; c <= Cfg::kMaxSplits; ++c) {
       clusters_of(c);
-      if (cudaOccupancyMaxActiveClusters(&active[c], kernel, &cfg) != cudaSuccess || active[c] <= 0) {
+      if (cudaOccupancyMaxActiveClusters(&active[c], kernel, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
-        return kAttnLaunchFailed;
+        active[c] = 0;  // a size this device cannot place
       }
     }
+    if (active[1] <= 0) return kAttnLaunchFailed;
     active_dev = dev;
   }
   clusters_of(split_count(units, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, active));
