@@ -24,7 +24,7 @@ from ..jit.compiler import get_default_user_dir, get_fray_version, put
 
 QUEUE_FLUSHES = 32     # 256 MB each, about 45 us: the host queues 20 launches in well under a millisecond
 LONG_LAUNCH_MS = 0.2   # from here on the host stays ahead by itself, and the board's power limit sets the clock
-ROUNDS = 2             # over all candidates; the last one counts
+HEAT_MS = 80           # of a candidate's own load, after which the clock has settled (0.93 ms a launch cold, 1.07-1.1 then)
 
 
 def _debug() -> bool:
@@ -70,8 +70,9 @@ class JITTuner:
         Differences from the reference: three untimed launches first (the first launch of a library pays module
         loading and the tensor-map encodings), and several timed batches.  Short launches: the best of three batches,
         each behind enough flushes to keep the device busy while the host queues it; marshalling a call takes longer
-        than a small kernel runs, and candidates of 10 to 20 us all measured the host's pace.  Long launches: the
-        middle one of three batches straight after one another, at the clock that this load leaves.
+        than a small kernel runs, and candidates of 10 to 20 us all measured the host's pace.  Long launches: one
+        batch straight behind enough of the same load to bring the board to the clock that it leaves; timed cold,
+        candidates rank by what ran before them.
         """
         for _ in range(3):
             assert runtime(*args) == 0
@@ -89,9 +90,11 @@ class JITTuner:
             end.synchronize()
             return start.elapsed_time(end) * launches / count
 
-        if batch(1, launches) < LONG_LAUNCH_MS * launches:
+        first = batch(1, launches)
+        if first < LONG_LAUNCH_MS * launches:
             return min(batch(QUEUE_FLUSHES, launches) for _ in range(3))
-        return sorted(batch(0, max(1, launches // 2)) for _ in range(3))[1]
+        batch(0, max(1, int(HEAT_MS * launches / first)))
+        return batch(0, launches)
 
     # ------------------------------------------------------------------ main entry
     def compile_and_tune(self, name: str, keys: Dict[str, Any], space: tuple, includes: tuple, arg_defs: tuple,
@@ -132,12 +135,7 @@ class JITTuner:
             elif _debug():
                 print(f"Illegal JIT kernel {name} with keys {keys} and tuned keys {tuned_keys}: "
                       f"error code {return_code}")
-        # The first round brings the board to the clock it keeps under this load and the last one counts: timed cold and
-        # one after the other, the candidates of a 1 ms problem rank by how early they are tried (0.93 ms in the first
-        # 30 ms, 1.13 after, for one and the same kernel).
-        times = [0.0] * len(legal)
-        for _ in range(ROUNDS if len(space) > 1 else 0):
-            times = [self.time_candidate(runtime, args) for runtime, _ in legal]
+        times = [self.time_candidate(runtime, args) if len(space) > 1 else 0.0 for runtime, _ in legal]
         best_runtime, best_time, best_keys = None, None, None
         for (runtime, tuned_keys), elapsed in zip(legal, times):
             if best_time is None or elapsed < best_time:
