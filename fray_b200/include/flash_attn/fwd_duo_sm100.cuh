@@ -66,7 +66,7 @@ struct DuoCfg {
   static constexpr int kOffKV = 2 * kQTileBytes;
   static constexpr int kOffStage = kOffKV + STAGES * kKVTileBytes;  // O staging tile behind the ring, for both query tiles
   static constexpr int kOffBars = kOffStage + kQTileBytes;
-  static constexpr int kNumBars = 2 * 2 + 2 * STAGES + 2 * 3 + 2 * kPChunks + 2;
+  static constexpr int kNumBars = 2 * 2 + 2 * STAGES + 2 * 3 + 2 * kPChunks + 3;
   static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // [2 tiles][2 halves][128]
   static constexpr int kUsedBytes = kOffStats + 4 * 128 * 4;
   // slack to bring the dynamic segment to a 1024-byte boundary (its base is one already; the kernel checks)
@@ -196,7 +196,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* o_free = o_full + 2;                // [2]   softmax i -> MMA (the item's O_i is in registers)
   uint64_t* p_full = o_free + 2;                // [2][kPChunks] softmax i -> MMA
   uint64_t* stage_full = p_full + 2 * Cfg::kPChunks;  // softmax -> store warp
-  uint64_t* stage_free = stage_full + 1;        // store warp -> softmax
+  uint64_t* stage_free = stage_full + 1;        // [2]   store warp -> softmax i (the staging tile is tile i's turn)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
   float* stats = reinterpret_cast<float*>(smem + Cfg::kOffStats);
@@ -263,6 +263,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     mbar_init(stage_full, 8);
     mbar_init(stage_free, 1);
+    mbar_init(stage_free + 1, 1);
     fence_barrier_init();
   }
   __syncwarp();
@@ -307,17 +308,14 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       tmem_wait_st();
     };
-    // phase parities, toggled: bit 0 s_full, bit 1 o_full, bits 2.. tiles of either index staged before
+    // phase parities, toggled: bit 0 s_full, bit 1 o_full, bit 2 stage_free
     uint32_t phases = 0;
     for (int k = 0, idx = pos(0); idx < total; idx = pos(++k)) {
       int n_i, row0;
-      uint32_t my_store;
       {
         const DuoItem it = decode(idx);
         n_i = i ? it.n1 : it.n0;
         row0 = it.m0 + i * Cfg::BM;
-        my_store = (phases >> 2) + (i && it.n0 > 0);
-        phases += 4u * ((it.n0 > 0) + (it.n1 > 0));
       }
       if (n_i == 0) continue;
       // the first steps see every key of their tile
@@ -346,7 +344,12 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       named_barrier_sync(pair_bar, 64);
       l_run += my_stat[other_off];
       named_barrier_sync(pair_bar, 64);  // the slots take the next item's maxima
-      if (my_store > 0) mbar_wait(stage_free, (my_store - 1) & 1, abort_flag, 0x321 + i, idx);
+      // The tile's turn at the staging buffer.  Each tile has a barrier of its own and meets every phase of it once: phase
+      // j completes when the store in front of the tile's j-th one has been read, and phase j + 1 not before the tile's
+      // j-th store, which needs all eight warps past this wait.  So the parity says whether phase j is complete whatever
+      // the store warp's delay; on one barrier for both tiles a wait could look over an open phase or miss two.
+      mbar_wait(stage_free + i, (phases >> 2) & 1, abort_flag, 0x321 + i, idx);
+      phases ^= 4u;
       mbar_wait(o_full + i, (phases >> 1) & 1, abort_flag, 0x331 + i, idx);
       phases ^= 2u;
       tc_fence_after_sync();
@@ -390,6 +393,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (warp == 18 && lane == 0) {
       // ============================================================= stores of finished tiles
       uint32_t stores = 0;
+      mbar_arrive(stage_free);  // the first store is a tile 0's (every item has one)
       for (int k = 0, idx = pos(0); idx < total; idx = pos(++k)) {
         const DuoItem it = decode(idx);
 #pragma unroll 1
@@ -402,7 +406,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             tma_store_4d(&tm_o, stage_smem + p * Cfg::kQPanelBytes, p * 64, it.m0 + i * Cfg::BM, it.h, it.b);
           tma_store_commit();
           tma_store_wait_read();
-          mbar_arrive(stage_free);
+          mbar_arrive(stage_free + (i == 0 && it.n1 > 0));  // whose store comes next: this item's tile 1, or an item's tile 0
           ++stores;
         }
       }

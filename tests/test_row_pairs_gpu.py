@@ -40,3 +40,39 @@ def test_row_pairs(B, H, Hkv, Sq, Sk, causal, D, gain, monkeypatch):
         assert (guard[b, :, :Sq].double() - torch.softmax(s, -1) @ ve).abs().max().item() <= 2 * 6 * 2.0 ** -11
         assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() <= 2e-4
         del s
+
+
+# Items of one or two KV steps over many rounds per CTA, both query tiles live, so that finished tiles follow each other
+# through the one staging buffer as fast as they can: every item two tiles; every third item without a second tile (rows
+# 512..599 of 600); a causal first tile of one step beside a second of two; ragged ends of both tiles.
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,causal", [
+    (4, 64, 64, 4096, 77, False), (3, 200, 50, 600, 100, False), (3, 200, 200, 256, 256, True), (2, 300, 300, 511, 128, False)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.half, torch.bfloat16])
+def test_finished_tiles_follow_each_other_closely(B, H, Hkv, Sq, Sk, causal, D, dtype, monkeypatch):
+    import importlib
+    op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
+    monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
+    point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
+    monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    g = torch.Generator(device="cuda").manual_seed(83)
+    q = torch.randn(B, H, Sq, D, generator=g, device="cuda").to(dtype)
+    k, v = (torch.randn(B, Hkv, Sk, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    outs = [torch.full((B, H, Sq, D), 7.0, dtype=dtype, device="cuda") for _ in range(4)]
+    for out in outs:
+        op.flash_attn_cute(q, k, v, out, causal=causal)
+    torch.cuda.synchronize()
+    assert op.flash_attn_status()[0] == 0
+    # P and the output are each rounded to 16 bits (within u of a value): a convex sum of |v| <= 6, as above
+    u = 2.0 ** -11 if dtype is torch.half else 2.0 ** -8
+    mask = torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril() if causal else None
+    for b in range(B):
+        ke, ve = (t[b].repeat_interleave(H // Hkv, 0).double() for t in (k, v))
+        s = q[b].double() @ ke.transpose(-1, -2) / math.sqrt(D)
+        if causal:
+            s.masked_fill_(~mask, float("-inf"))
+        want = torch.softmax(s, -1) @ ve
+        assert (outs[0][b].double() - want).abs().max().item() <= 2 * 6 * u
+        del s, want
+    for out in outs[1:]:
+        assert torch.equal(out, outs[0])
