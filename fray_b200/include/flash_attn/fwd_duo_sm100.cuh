@@ -340,10 +340,12 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           phases ^= 1u;
         }
       }
+      // The slots carried maxima up to the last step, whose exchange ends with a read of the partner's: both warps have to
+      // be past it before a row sum takes a maximum's place.
+      named_barrier_sync(pair_bar, 64);
       *my_stat = l_run;
       named_barrier_sync(pair_bar, 64);
-      l_run += my_stat[other_off];
-      named_barrier_sync(pair_bar, 64);  // the slots take the next item's maxima
+      l_run += my_stat[other_off];  // the next write to a slot comes behind the next step's OR barrier
       // The tile's turn at the staging buffer.  Each tile has a barrier of its own and meets every phase of it once: phase
       // j completes when the store in front of the tile's j-th one has been read, and phase j + 1 not before the tile's
       // j-th store, which needs all eight warps past this wait.  So the parity says whether phase j is complete whatever

@@ -76,3 +76,30 @@ def test_finished_tiles_follow_each_other_closely(B, H, Hkv, Sq, Sk, causal, D, 
         del s, want
     for out in outs[1:]:
         assert torch.equal(out, outs[0])
+
+
+# One step per item: the exchange of maxima and that of row sums use the same slots with nothing but one step's arithmetic in
+# between; a half that took the partner's row sum for its maximum would show in the row sum and in half of the row's weights.
+@pytest.mark.parametrize("Sq,Sk", [(512, 128), (513, 65), (256, 127)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_halves_of_a_row_agree_in_items_of_one_step(Sq, Sk, D, monkeypatch):
+    import importlib
+    op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
+    monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
+    point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
+    monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    g = torch.Generator(device="cuda").manual_seed(89)
+    B, H = 4, 150
+    q = (6.0 * torch.randn(B, H, Sq, D, generator=g, device="cuda")).half()
+    k, v = (torch.randn(B, H, Sk, D, generator=g, device="cuda").half() for _ in range(2))
+    out, lse = torch.zeros_like(q), torch.zeros(B, H, Sq, device="cuda")
+    for _ in range(4):
+        op.flash_attn_cute(q, k, v, out, lse=lse)
+    torch.cuda.synchronize()
+    assert op.flash_attn_status()[0] == 0
+    for b in range(B):
+        s = q[b].double() @ k[b].double().transpose(-1, -2) / math.sqrt(D)
+        # bounds as in test_row_pairs
+        assert (out[b].double() - torch.softmax(s, -1) @ v[b].double()).abs().max().item() <= 2 * 6 * 2.0 ** -11
+        assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() <= 2e-4
+        del s
