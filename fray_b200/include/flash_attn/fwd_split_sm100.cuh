@@ -12,8 +12,9 @@
 //     workspace, no second launch and no order between clusters;
 //   * a tile of up to 32 rows is placed four times (up to 64: twice) in the 128-row operand, and the warps, each of which
 //     reaches only its own 32 lanes of tensor memory, each take a quarter (half) of a step's keys for the same rows: the
-//     P of the other keys stays zero, the copies' partial sums are merged with the splits'.  The warps share nothing
-//     inside a step, and a step's exponentials take a quarter of the time;
+//     products of a copy's keys write that copy's lanes only (a zero P would do for finite V, but 0 x Inf is NaN), the
+//     copies' partial sums are merged with the splits'.  The warps share nothing inside a step, and a step's exponentials
+//     take a quarter of the time;
 //   * scores and probabilities have two tensor-memory buffers each, so S(t+2) is issued behind P.V(t) and the
 //     tensor pipe never waits for a softmax of its own step.
 //
@@ -138,14 +139,6 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t t_o = tmem_base + Cfg::kColO + lane_base;
     const int slot = warp * 32 + lane;
     const bool mine = slot % kRowsPerCopy < rows;  // the other lanes' rows hold whatever shared memory held
-    if (COPIES > 1) {  // P of the keys other copies take: zero, and nothing writes there again
-      uint32_t z[16];
-#pragma unroll
-      for (int x = 0; x < 16; ++x) z[x] = 0u;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) tmem_st_x16(tmem_base + Cfg::kColP + c * 16 + lane_base, z);
-      tmem_wait_st();
-    }
     float m_ref = -INFINITY, l_run = 0.f;
     for (int t = 0; t < n; ++t) {
       const uint32_t t_s = tmem_base + Cfg::kColS + (t & 1) * 128 + lane_base;
@@ -295,9 +288,18 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tc_fence_after_sync();
       const uint32_t v_lo = static_cast<uint32_t>(kDescV) | (((kv_addr + slot * Cfg::kKVTileBytes) & 0x3FFFF) >> 4);
 #pragma unroll
-      for (int kk = 0; kk < BN / 16; ++kk)
-        mma_ts_elect_lohi(tmem_base + Cfg::kColO, tmem_base + Cfg::kColP + (t & 1) * 64 + kk * 8, v_lo + ((kk * 2048) >> 4),
-                          kDescVHi, kIdescPV, (t > 0 || kk > 0));
+      for (int kk = 0; kk < BN / 16; ++kk) {  // 16 keys each
+        const uint32_t t_p = tmem_base + Cfg::kColP + (t & 1) * 64 + kk * 8;
+        const uint32_t v_kk = v_lo + ((kk * 2048) >> 4);
+        if constexpr (COPIES == 1) {
+          mma_ts_elect_lohi(tmem_base + Cfg::kColO, t_p, v_kk, kDescVHi, kIdescPV, (t > 0 || kk > 0));
+        } else {
+          constexpr int kPerCopy = BN / 16 / COPIES;
+          auto keep = [&](int w) { return w * COPIES / 4 == kk / kPerCopy ? 0u : ~0u; };  // other copies' lanes stay
+          mma_ts_elect_lohi_lanes(tmem_base + Cfg::kColO, t_p, v_kk, kDescVHi, kIdescPV, (t > 0 || kk % kPerCopy > 0), keep(0),
+                                  keep(1), keep(2), keep(3));
+        }
+      }
       mma_commit_elect(o_full);
       mma_commit_elect(kv_empty + slot);
       ++c;

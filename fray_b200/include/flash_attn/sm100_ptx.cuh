@@ -328,6 +328,24 @@ __device__ __forceinline__ void mma_ts_elect_lohi(uint32_t d_tmem, uint32_t a_tm
       : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with a mask of accumulator lanes that are left as they are (bit x of keep_w: lane 32 * w + x).
+__device__ __forceinline__ void mma_ts_elect_lohi_lanes(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi,
+                                                        uint32_t idesc, uint32_t accumulate, uint32_t keep_0, uint32_t keep_1,
+                                                        uint32_t keep_2, uint32_t keep_3) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, e;\n"
+      ".reg .b64 db;\n"
+      "mov.b64 db, {%2, %3};\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, {%6, %7, %8, %9}, p;\n"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(keep_0), "r"(keep_1), "r"(keep_2),
+        "r"(keep_3)
+      : "memory");
+}
 __device__ __forceinline__ void mma_commit_elect(uint64_t* bar) {
   asm volatile(
       "{\n"

@@ -57,3 +57,30 @@ def test_few_queries_non_finite_values_stay_in_their_rows():
     assert torch.isnan(out[0, 2, 1]).all()
     out[0, 2, 1] = want[0, 2, 1]
     assert torch.equal(out, want)
+
+
+# every row placement (rows = 4, 32, 44, 64, 100) and infinities in every quarter of a step, in several splits and in the
+# ragged last step: a key's value reaches the sums of its own weights only, never a product with another copy's zero
+@pytest.mark.parametrize("H,Sq", [(4, 1), (4, 8), (4, 11), (4, 16), (4, 25)])
+@pytest.mark.parametrize("Sk", [600, 3000])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.half, torch.bfloat16])
+def test_few_queries_infinite_values_stay_in_their_columns(H, Sq, Sk, D, dtype):
+    from fray_b200.jit_kernels import flash_attn_cute, flash_attn_status
+    g = torch.Generator(device="cuda").manual_seed(79)
+    q, k, v = (torch.randn(2, h, s, D, generator=g, device="cuda").to(dtype) for h, s in ((H, Sq), (1, Sk), (1, Sk)))
+    want = torch.zeros_like(q)
+    flash_attn_cute(q, k, v, want)
+    for column, key in enumerate((5, 40, 70, 101, 300, 511, Sk - 1)):
+        v[0, 0, key, 3 * column] = float("inf")
+        v[0, 0, key, 3 * column + 1] = float("-inf")
+        want[0, :, :, 3 * column] = float("inf")  # weights of normal scores stay above the smallest 16-bit number
+        want[0, :, :, 3 * column + 1] = float("-inf")
+    v[0, 0, 200, 40], v[0, 0, 330, 40], v[0, 0, 450, 41] = float("inf"), float("-inf"), float("nan")
+    want[0, :, :, 40:42] = float("nan")
+    out = torch.zeros_like(q)
+    flash_attn_cute(q, k, v, out)
+    torch.cuda.synchronize()
+    assert flash_attn_status()[0] == 0
+    no_number = torch.isnan(want)
+    assert torch.equal(torch.isnan(out), no_number) and torch.equal(out[~no_number], want[~no_number])
