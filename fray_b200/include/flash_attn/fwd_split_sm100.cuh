@@ -198,6 +198,10 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         exp_32(s[c], scale2, neg_m2, rsp0, rsp1, pk);
         tmem_st_x16(t_p + (c0 + c) * 16, pk);
       }
+      // The epilogue waits for P.V(n-1) by parity, so P.V(n-2) has to be known complete by then: S(n-1) was issued ahead of it
+      // and says so of P.V(n-3) only.  Met here, where P.V(n-1) cannot complete before this warp's P; behind the hand-over a
+      // held-up warp could miss it and wait for a phase that never comes.
+      if (t > 0 && t == n - 1) mbar_wait(o_full, (t - 1) & 1, abort_flag, 0x330, t);
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
@@ -208,8 +212,6 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       l_run += (r0 + r1) + (r2 + r3);
     }
     if (n > 0) {
-      // S(n-1) may be complete before P.V(n-2) is: pass that phase first, or the last one's parity would look over
-      if (n > 1) mbar_wait(o_full, (n - 2) & 1, abort_flag, 0x330, n);
       mbar_wait(o_full, (n - 1) & 1, abort_flag, 0x331, n);
       tc_fence_after_sync();
       // Every copy into the ring has been read by a completed product: the partial results take its place.
