@@ -91,14 +91,13 @@ _RC_TENSOR_MAP = 6
 KIND_SIMPLE, KIND_TWO_TILES, KIND_ALTERNATING, KIND_PAIRED, KIND_ONE_TILE = 0, 1, 2, 3, 4
 KIND_FEW_QUERIES, KIND_ROW_PAIRS = 6, 7
 
-# The few-query kernel holds all rows (queries x query heads per K/V head) of a K/V head in one 128-row tile.
+# The few-query kernel holds all rows (queries x query heads per K/V head) of a K/V head in one 128-row tile.  Up to half
+# that many are placed several times, and its warps share out the keys of a step.
 FEW_QUERY_ROWS = 128
+FEW_QUERY_SHARED_STEP_ROWS = 64
 # Below this many keys its cluster's start and merge cost more than the split saves (16 heads x 128 queries, head dim
 # 128: 11.2 us against 7.3 at 256 keys, 9.5 against 10.8 at 512, 10.6 against 17.2 at 1024).
 FEW_QUERY_MIN_KEYS = 512
-# With a K/V head per query head there are no rows to share, and once the units fill the chip by themselves only long
-# units gain (1024 units: 61 us against 51 at 512 keys, 92 against 90 at 1024, 185 against 228 at 4096).
-FEW_QUERY_LONG_KEYS = 4096
 
 
 def few_query_space() -> Tuple[Dict[str, Any], ...]:
@@ -107,13 +106,35 @@ def few_query_space() -> Tuple[Dict[str, Any], ...]:
     return ({"KIND": KIND_FEW_QUERIES, "BLOCK_N": 128, "STAGES": 4},)
 
 
-def _few_queries(group: int, seq_len: int, seq_len_kv: int, causal: bool, units: int, sms: int) -> bool:
+def _few_queries(group: int, seq_len: int, seq_len_kv: int, causal: bool, units: int, sms: int, d: int = 128) -> bool:
     """Whether a call goes to the few-query kernel: all rows of a K/V head's group fit one tile, every row sees every
-    key and there are many keys (a decoding step, a short chunk of new queries).  Such a call is bound by reading K and V
-    once, not by arithmetic.  ``units``: batch x K/V heads."""
-    if causal or group * seq_len > FEW_QUERY_ROWS or seq_len_kv < FEW_QUERY_MIN_KEYS:
+    key, there are many keys (a decoding step, a short chunk of new queries), and the kernel is no slower there than the
+    best of the others.  ``units``: batch x K/V heads.
+
+    It gains in two ways: the query heads of a group share one reading of K and V, and while two and more CTAs per unit fit
+    the chip they share its keys.  Figures: its time over the best other kernel's, on 148 SMs, for 5100 combinations of 4 to
+    1000 units, groups of 1 to 8, 1 to 128 rows and 512 to 8192 keys at both head dims: 0.11 to 1.03 where it is taken.
+    """
+    rows = group * seq_len
+    if causal or rows > FEW_QUERY_ROWS or seq_len_kv < FEW_QUERY_MIN_KEYS:
         return False
-    return group > 1 or units <= sms or seq_len_kv >= FEW_QUERY_LONG_KEYS
+    if rows <= FEW_QUERY_SHARED_STEP_ROWS:
+        if group > 1 or 2 * units <= sms:  # 0.11-1.01
+            return True
+        # Nothing is shared and no unit's keys are split: only a step that is short beside its copies gains.
+        if units <= sms:  # 32 rows: 0.62-1.00 at head dim 64, 0.64-0.94 up to 1024 keys, beyond that up to 1.13 (4 rows: 1.02)
+            return rows <= (32 if d == 64 or seq_len_kv <= 1024 else 4)
+        # One whole-SM CTA per unit pays for its start and end on top, and for an incomplete last round: 16 rows, 150 units:
+        # 1.11 at 4096 keys and 0.92 at 8192 (head dim 64: 0.88, 0.66), 300 units: 0.87 at 4096.
+        return rows <= 16 and seq_len_kv >= (4096 if d == 64 or units >= 2 * sms else 8192)
+    # A warp goes through all 128 keys of a step for its rows, as in the one-tile kernels that have two CTAs per SM.
+    if group >= 4 and group * units > sms:  # the others need a round and more per head of a group: 0.16-1.02
+        return True
+    if 2 * units <= sms:  # keys split; 512 keys: 0.78-0.92 at 16 units, 1.2 at 37 (768: 0.92); 60 units 1.10 at 768, 1.03 at 1024
+        return seq_len_kv >= (512 if 8 * units <= sms else 768 if 4 * units <= sms else 1024)
+    if group == 1:  # 0.94-2.36
+        return False
+    return seq_len_kv >= (1536 if group == 2 else 1024)  # 2 x 64 rows: 1.44 at 512 keys, 1.20 at 1024, 1.03 at 1536
 
 
 def tuning_space(d: int) -> Tuple[Dict[str, Any], ...]:
@@ -321,7 +342,7 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
     args = pack(q, k, v, out)
     forced = os.getenv("FRAY_ATTN_FORCE", "")
     few = not forced and _few_queries(num_heads // num_kv_heads, seq_len, seq_len_kv, bool(causal), batch_size * num_kv_heads,
-                                           torch.cuda.get_device_properties(Q.device).multi_processor_count)
+                                      torch.cuda.get_device_properties(Q.device).multi_processor_count, d)
     runtime = jit_tuner.compile_and_tune(
         name="flash_attn_cute",
         keys={"D": d, "CAUSAL": int(bool(causal)),

@@ -20,7 +20,8 @@ def exact(q, k, v):
 @pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D,gain", [
     (1, 1, 1, 1, 512, 64, 1.0), (1, 4, 1, 1, 513, 128, 1.0), (1, 8, 1, 4, 639, 128, 4.0), (2, 3, 1, 11, 1025, 64, 4.0),
     (1, 4, 2, 32, 4096, 128, 4.0), (2, 5, 1, 13, 1000, 128, 1.0), (1, 1, 1, 127, 515, 64, 4.0), (1, 2, 1, 64, 2049, 128, 4.0),
-    (80, 4, 2, 1, 600, 64, 4.0), (8, 32, 8, 1, 8192, 128, 1.0), (1, 16, 2, 8, 16000, 128, 6.0)])
+    (80, 4, 2, 1, 600, 64, 4.0), (8, 32, 8, 1, 8192, 128, 1.0), (1, 16, 2, 8, 16000, 128, 6.0),
+    (40, 8, 2, 25, 700, 64, 4.0)])
 @pytest.mark.parametrize("dtype", [torch.half, torch.bfloat16])
 def test_few_queries(B, H, Hkv, Sq, Sk, D, gain, dtype):
     from fray_b200.jit_kernels import flash_attn_cute, flash_attn_status
