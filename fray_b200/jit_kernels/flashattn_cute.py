@@ -179,10 +179,12 @@ def _forced_point() -> Optional[Dict[str, int]]:
     return point
 
 
-def _seq_class(seq_len: int, units: int) -> str:
-    """Coarse workload class the tuner memoises on: sequence bucket and whether the grid fills the GPU."""
-    s_bucket = 1 << max(7, (max(seq_len, 1) - 1).bit_length())
-    return f"S{min(s_bucket, 16384)}_{'big' if units * seq_len >= 148 * 256 else 'small'}"
+def _workload_class(seq_len: int, seq_len_kv: int, units: int, sms: int) -> str:
+    """Coarse workload class the tuner memoises on, from what the kinds differ in: how many steps a work item has (bucket of
+    the number of keys), whether items of two query tiles fill the chip, and whether there is a second tile at all."""
+    k_bucket = 1 << max(7, (max(seq_len_kv, 1) - 1).bit_length())
+    fill = "big" if units * -(-seq_len // 256) >= sms else "small"
+    return f"K{min(k_bucket, 16384)}_{fill}{'_one_tile' if seq_len <= 128 else ''}"
 
 
 def _usable_strides(t: torch.Tensor) -> bool:
@@ -341,12 +343,13 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
 
     args = pack(q, k, v, out)
     forced = os.getenv("FRAY_ATTN_FORCE", "")
+    sms = torch.cuda.get_device_properties(Q.device).multi_processor_count
     few = not forced and _few_queries(num_heads // num_kv_heads, seq_len, seq_len_kv, bool(causal), batch_size * num_kv_heads,
-                                      torch.cuda.get_device_properties(Q.device).multi_processor_count, d)
+                                      sms, d)
     runtime = jit_tuner.compile_and_tune(
         name="flash_attn_cute",
         keys={"D": d, "CAUSAL": int(bool(causal)),
-              "CLASS": "few" if few else _seq_class(max(seq_len, seq_len_kv), batch_size * num_heads),
+              "CLASS": "few" if few else _workload_class(seq_len, seq_len_kv, batch_size * num_heads, sms),
               "FORCED": forced, **({"BF16": 1} if bf16 else {})},
         space=few_query_space() if few else tuning_space(d),
         includes=includes_bf16 if bf16 else includes,

@@ -62,6 +62,17 @@ def test_tuning_space_varies_tile_rows_stages_and_cta_pairing(monkeypatch):
     assert op.KIND_PAIRED not in {p["KIND"] for p in op.tuning_space(64)}
 
 
+def test_workload_classes_tell_query_tiles_from_keys():
+    cls = op._workload_class
+    # one verdict for all of these would make speed depend on which call came first
+    chunk, square, decode, cross = (cls(513, 6000, 32, 148), cls(6000, 6000, 32, 148), cls(1, 6000, 32, 148), cls(4096, 77, 32, 148))
+    assert len({chunk, square, decode, cross}) == 4
+    assert cls(6000, 6000, 32, 148) == cls(8192, 8192, 32, 148) == cls(5000, 4097, 128, 148)   # a bucket is a power of two of keys
+    assert cls(256, 4096, 148, 148) != cls(256, 4096, 147, 148)                                # items of 256 rows against the SMs
+    assert cls(128, 4096, 500, 148) != cls(129, 4096, 500, 148)                                # a second query tile or none
+    assert cls(40000, 40000, 32, 148) == cls(16384, 16384, 32, 148) and cls(1, 1, 1, 148) == cls(64, 128, 1, 148)
+
+
 def test_prebuild_point_list_keeps_the_whole_space_when_a_point_is_forced(monkeypatch):
     monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
     whole = op._space_points((64, 128), forced=False)
