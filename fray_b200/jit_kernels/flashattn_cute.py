@@ -181,11 +181,9 @@ def _forced_point() -> Optional[Dict[str, int]]:
 
 def _workload_class(seq_len: int, seq_len_kv: int, units: int, sms: int) -> str:
     """Coarse workload class the tuner memoises on, from what the kinds differ in: how many steps a work item has (bucket of
-    the number of keys), whether items of two query tiles fill the chip, most of it or a corner (64-wide causal heads of 333
-    rows: kind 7 9.7 us, kind 4 10.8 at 144 items; 256 rows, 4 items: 8.5 and 6.0), and whether there is a second tile."""
+    the number of keys), whether items of two query tiles fill the chip, and whether there is a second tile at all."""
     k_bucket = 1 << max(7, (max(seq_len_kv, 1) - 1).bit_length())
-    items = units * -(-seq_len // 256)
-    fill = "big" if items >= sms else "part" if 4 * items >= sms else "small"
+    fill = "big" if units * -(-seq_len // 256) >= sms else "small"
     return f"K{min(k_bucket, 16384)}_{fill}{'_one_tile' if seq_len <= 128 else ''}"
 
 
