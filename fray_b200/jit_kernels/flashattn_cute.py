@@ -11,6 +11,7 @@ consumed and produced through their strides (no hidden copies, and a non-contigu
 import ctypes
 import math
 import os
+import threading
 from collections import OrderedDict
 from typing import Any, Dict, Optional, Tuple
 
@@ -381,7 +382,21 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
         Output.copy_(out)
 
 
+# Device staging buffers of the host-buffer call, one shape at a time, shared by every stream and thread of the process: the
+# events say until when a buffer set is in use, the lock covers the queueing of a whole call.
 _host_staging: Dict[Any, Any] = {}
+_host_staging_lock = threading.Lock()
+
+
+def _drop_host_staging() -> None:
+    """Gives the staging buffers back once everything queued on them, on whatever stream, has run."""
+    for st in _host_staging.values():
+        for event in (*st["computed"], *st["drained"]):
+            if event is not None:
+                st["s_in"].wait_event(event)
+        for buf in (*st["bufs"][0], *st["bufs"][1]):
+            buf.record_stream(st["s_in"])
+    _host_staging.clear()
 
 
 def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: torch.Tensor, *,
@@ -398,7 +413,8 @@ def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Outp
     directions of the host link run at the same time and the kernel hides behind them.  Work is ordered
     after the current stream's earlier work, and the current stream waits for the last copy-out: as with the
     device op, the result is valid for work queued on the current stream afterwards (or after a
-    synchronize), not at return.
+    synchronize), not at return.  Calls may come from several streams and threads: they share the staging
+    buffers, one after the other on the device, and queue one at a time; a captured call has its own.
     """
     tensors = (Q, K, V, Output) + ((lse,) if lse is not None else ())
     assert all(t.device.type == "cpu" and t.is_pinned() for t in tensors), "operands must be pinned host tensors"
@@ -420,52 +436,60 @@ def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Outp
     bounds = [(units * c) // n for c in range(n + 1)]
     rows = max(b1 - b0 for b0, b1 in zip(bounds, bounds[1:]))
     key = (dev, rows, group, Sq, Sk, D, Q.dtype, lse is not None)
-    st = _host_staging.get(key)
-    if st is None:
-        def make_set():
-            bufs = [torch.empty((rows, group, Sq, D), dtype=Q.dtype, device=dev),
-                    torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
-                    torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
-                    torch.empty((rows, group, Sq, D), dtype=Q.dtype, device=dev)]
-            if lse is not None:
-                bufs.append(torch.empty((rows, group, Sq), dtype=torch.float32, device=dev))
-            return bufs
-        st = {"bufs": [make_set(), make_set()], "s_in": torch.cuda.Stream(device=dev), "s_out": torch.cuda.Stream(device=dev)}
-        _host_staging.clear()  # one shape at a time: the buffers are as large as the operands' slices
-        _host_staging[key] = st
-    s_in, s_out = st["s_in"], st["s_out"]
-    cur = torch.cuda.current_stream(dev)
-    start = torch.cuda.Event()
-    start.record(cur)
-    s_in.wait_event(start)
-    s_out.wait_event(start)
-    computed = [None, None]   # per buffer set: kernel of the slice that last used it has finished
-    drained = [None, None]    # ... and its result has left the device
-    for c, (b0, b1) in enumerate(zip(bounds, bounds[1:])):
-        bufs = [t[: b1 - b0] for t in st["bufs"][c & 1]]
-        dq, dk, dv, do = bufs[:4]
-        if computed[c & 1] is not None:
-            s_in.wait_event(computed[c & 1])      # inputs of slice c-2 are no longer read
-        with torch.cuda.stream(s_in):
-            dq.copy_(Qu[b0:b1], non_blocking=True)
-            dk.copy_(Ku[b0:b1], non_blocking=True)
-            dv.copy_(Vu[b0:b1], non_blocking=True)
-            arrived = torch.cuda.Event()
-            arrived.record(s_in)
-        cur.wait_event(arrived)
-        if drained[c & 1] is not None:
-            cur.wait_event(drained[c & 1])        # output buffers of slice c-2 have been copied out
-        # a slice is itself an attention problem with batch = units in the slice, H = group, H_kv = 1
-        flash_attn_cute(dq, dk, dv, do, causal=causal, scale=scale, lse=bufs[4] if lse is not None else None)
-        computed[c & 1] = torch.cuda.Event()
-        computed[c & 1].record(cur)
-        s_out.wait_event(computed[c & 1])
-        with torch.cuda.stream(s_out):
-            Ou[b0:b1].copy_(do, non_blocking=True)
-            if lse is not None:
-                Lu[b0:b1].copy_(bufs[4], non_blocking=True)
-            drained[c & 1] = torch.cuda.Event()
-            drained[c & 1].record(s_out)
-    for ev in drained:
-        if ev is not None:
-            cur.wait_event(ev)
+    with _host_staging_lock:
+        # A graph being captured gets buffers of its own (from its pool): it runs whenever it is replayed, and events of calls
+        # outside it cannot be waited for in it.
+        capturing = torch.cuda.is_current_stream_capturing()
+        st = None if capturing else _host_staging.get(key)
+        if st is None:
+            def make_set():
+                bufs = [torch.empty((rows, group, Sq, D), dtype=Q.dtype, device=dev),
+                        torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
+                        torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
+                        torch.empty((rows, group, Sq, D), dtype=Q.dtype, device=dev)]
+                if lse is not None:
+                    bufs.append(torch.empty((rows, group, Sq), dtype=torch.float32, device=dev))
+                return bufs
+            if not capturing:
+                _drop_host_staging()  # one shape at a time: the buffers are as large as the operands' slices
+            st = {"bufs": [make_set(), make_set()], "s_in": torch.cuda.Stream(device=dev), "s_out": torch.cuda.Stream(device=dev),
+                  "computed": [None, None],   # per buffer set: kernel of the slice that last used it has finished
+                  "drained": [None, None]}    # ... and its result has left the device
+            if not capturing:
+                _host_staging[key] = st
+        s_in, s_out = st["s_in"], st["s_out"]
+        # Kept from call to call: a call on another stream finds the sets still in use by the one before it.
+        computed, drained = st["computed"], st["drained"]
+        cur = torch.cuda.current_stream(dev)
+        start = torch.cuda.Event()
+        start.record(cur)
+        s_in.wait_event(start)
+        s_out.wait_event(start)
+        for c, (b0, b1) in enumerate(zip(bounds, bounds[1:])):
+            bufs = [t[: b1 - b0] for t in st["bufs"][c & 1]]
+            dq, dk, dv, do = bufs[:4]
+            if computed[c & 1] is not None:
+                s_in.wait_event(computed[c & 1])      # inputs of slice c-2 are no longer read
+            with torch.cuda.stream(s_in):
+                dq.copy_(Qu[b0:b1], non_blocking=True)
+                dk.copy_(Ku[b0:b1], non_blocking=True)
+                dv.copy_(Vu[b0:b1], non_blocking=True)
+                arrived = torch.cuda.Event()
+                arrived.record(s_in)
+            cur.wait_event(arrived)
+            if drained[c & 1] is not None:
+                cur.wait_event(drained[c & 1])        # output buffers of slice c-2 have been copied out
+            # a slice is itself an attention problem with batch = units in the slice, H = group, H_kv = 1
+            flash_attn_cute(dq, dk, dv, do, causal=causal, scale=scale, lse=bufs[4] if lse is not None else None)
+            computed[c & 1] = torch.cuda.Event()
+            computed[c & 1].record(cur)
+            s_out.wait_event(computed[c & 1])
+            with torch.cuda.stream(s_out):
+                Ou[b0:b1].copy_(do, non_blocking=True)
+                if lse is not None:
+                    Lu[b0:b1].copy_(bufs[4], non_blocking=True)
+                drained[c & 1] = torch.cuda.Event()
+                drained[c & 1].record(s_out)
+        for ev in drained:
+            if ev is not None:
+                cur.wait_event(ev)

@@ -1,0 +1,154 @@
+"""Order of the host-buffer call's work on its shared staging buffers: streams and events are faked with logical clocks, every
+access to a buffer is recorded, and any two of which one writes have to be ordered."""
+import contextlib
+import importlib
+import threading
+
+import pytest
+import torch
+
+op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
+
+
+alive = []  # identities and addresses stay apart
+
+
+class FakeStream:
+    def __init__(self, device=None):
+        self.clock = {}
+        alive.append(self)
+
+    def tick(self):
+        self.clock[id(self)] = self.clock.get(id(self), 0) + 1
+        return id(self), dict(self.clock)
+
+    def wait_event(self, event):
+        for k, v in event.clock.items():
+            self.clock[k] = max(self.clock.get(k, 0), v)
+
+
+class FakeEvent:
+    def __init__(self, *a, **k):
+        self.clock = {}
+
+    def record(self, stream):
+        self.clock = dict(stream.clock)
+
+
+def before(a, b):
+    return a[1][a[0]] <= b[1].get(a[0], 0)
+
+
+@pytest.fixture
+def device(monkeypatch):
+    """Runs flash_attn_cute_host on the CPU; returns (set_current, accesses, released)."""
+    accesses, released = [], []
+    state = threading.local()
+    state.current = FakeStream()
+    empty, copy_ = torch.empty, torch.Tensor.copy_
+
+    def buffer_of(t):
+        return t.untyped_storage().data_ptr()
+
+    def log(t, write):
+        accesses.append((buffer_of(t), write, state.current.tick()))
+
+    def fake_empty(*a, device=None, **k):
+        t = empty(*a, **k)
+        alive.append(t)
+        return t
+
+    def fake_copy(dst, src, non_blocking=False):
+        log(src, False)
+        log(dst, True)
+        return copy_(dst, src)
+
+    @contextlib.contextmanager
+    def use(stream):
+        old, state.current = state.current, stream
+        try:
+            yield
+        finally:
+            state.current = old
+
+    def kernel(q, k, v, o, causal=False, scale=None, lse=None):
+        for t in (q, k, v):
+            log(t, False)
+        log(o, True)
+        if lse is not None:
+            log(lse, True)
+
+    monkeypatch.setattr(torch, "empty", fake_empty)
+    monkeypatch.setattr(torch.Tensor, "copy_", fake_copy)
+    monkeypatch.setattr(torch.Tensor, "is_pinned", lambda self: True)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, s: released.append((buffer_of(self), s.tick())))
+    monkeypatch.setattr(torch.cuda, "Stream", FakeStream)
+    monkeypatch.setattr(torch.cuda, "Event", FakeEvent)
+    monkeypatch.setattr(torch.cuda, "stream", use)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: state.current)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(op, "flash_attn_cute", kernel)
+    monkeypatch.setattr(op, "_host_staging", {})
+    return use, accesses, released
+
+
+def operands(B, S, lse):
+    t = [torch.zeros(B, 2, S, 64, dtype=torch.half) for _ in range(4)]
+    l = torch.zeros(B, 2, S) if lse else None
+    alive.extend((*t, l))
+    return t, l
+
+
+def unordered(accesses):
+    return [(a, b) for n, a in enumerate(accesses) for b in accesses[:n]
+            if a[0] == b[0] and (a[1] or b[1]) and not (before(a[2], b[2]) or before(b[2], a[2]))]
+
+
+@pytest.mark.parametrize("lse", [False, True])
+@pytest.mark.parametrize("chunks", [1, 2, 3, 8])
+def test_calls_on_other_streams_wait_for_the_buffers(device, lse, chunks):
+    use, accesses, _ = device
+    for stream in (FakeStream(), FakeStream(), FakeStream()):  # nothing orders the callers' streams
+        t, l = operands(4, 16, lse)
+        with use(stream):
+            op.flash_attn_cute_host(*t, lse=l, chunks=chunks)
+    assert accesses and not unordered(accesses)
+
+
+def test_buffers_are_given_back_after_their_last_use(device):
+    use, accesses, released = device
+    for S in (16, 24):
+        for stream in (FakeStream(), FakeStream()):
+            t, _ = operands(3, S, False)
+            with use(stream):
+                op.flash_attn_cute_host(*t, chunks=3)
+    assert len(released) == 8 and len(op._host_staging) == 1
+    for buf, stamp in released:
+        uses = [a for a in accesses if a[0] == buf]
+        assert uses and all(before(a[2], stamp) for a in uses)
+    assert not unordered(accesses)
+
+
+def test_one_call_queues_at_a_time(device, monkeypatch):
+    """Threads with one shape: their work on the shared buffers is not interleaved."""
+    inside, most = [0], [0]
+
+    def kernel(*a, **k):
+        inside[0] += 1
+        most[0] = max(most[0], inside[0])
+        threading.Event().wait(0.02)
+        inside[0] -= 1
+
+    main = torch.cuda.current_stream()
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: main)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(torch.Tensor, "copy_", lambda dst, src, non_blocking=False: dst)
+    monkeypatch.setattr(op, "flash_attn_cute", kernel)
+    calls = [operands(2, 8, False)[0] for _ in range(3)]
+    threads = [threading.Thread(target=lambda t=t: op.flash_attn_cute_host(*t, chunks=2)) for t in calls]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert most[0] == 1
