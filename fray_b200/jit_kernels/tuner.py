@@ -68,11 +68,11 @@ class JITTuner:
         """Milliseconds for ``launches`` back-to-back calls after an L2 flush (reference: tuner.py:52-63).
 
         Differences from the reference: three untimed launches first (the first launch of a library pays module
-        loading and the tensor-map encodings), and several timed batches.  Short launches: the best of three batches,
-        each behind enough flushes to keep the device busy while the host queues it; marshalling a call takes longer
-        than a small kernel runs, and candidates of 10 to 20 us all measured the host's pace.  Long launches: one
-        batch straight behind enough of the same load to bring the board to the clock that it leaves; timed cold,
-        candidates rank by what ran before them.
+        loading and the tensor-map encodings), and the best of three timed batches, so that one slow batch does not
+        drop a candidate.  Short launches: each batch behind enough flushes to keep the device busy while the host
+        queues it; marshalling a call takes longer than a small kernel runs, and candidates of 10 to 20 us all measured
+        the host's pace.  Long launches: straight behind enough of the same load to bring the board to the clock that it
+        leaves; timed cold, candidates rank by what ran before them.
         """
         for _ in range(3):
             assert runtime(*args) == 0
@@ -94,7 +94,7 @@ class JITTuner:
         if first < LONG_LAUNCH_MS * launches:
             return min(batch(QUEUE_FLUSHES, launches) for _ in range(3))
         batch(0, max(1, int(HEAT_MS * launches / first)))
-        return batch(0, launches)
+        return min(batch(0, launches) for _ in range(3))
 
     # ------------------------------------------------------------------ main entry
     def compile_and_tune(self, name: str, keys: Dict[str, Any], space: tuple, includes: tuple, arg_defs: tuple,

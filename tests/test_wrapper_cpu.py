@@ -141,6 +141,30 @@ def test_tuner_picks_fastest_legal_candidate_and_memoises(monkeypatch, tmp_path)
     assert t2.compile_and_tune("k", {"D": 128}, space, (), (), "k<{T}>", args=()) is table["k<1>"]
 
 
+@pytest.mark.parametrize("batches", [[90.0, 800.0, 50.0, 40.0, 45.0], [90.0, 800.0, 40.0, 70.0, 41.0],  # first, heating, three timed
+                                     [2.0, 1.9, 1.2, 1.5]])                                              # first, three timed
+def test_one_slow_batch_does_not_drop_a_candidate(monkeypatch, batches):
+    times = iter(batches)
+
+    class Event:
+        def __init__(self, enable_timing=False):
+            pass
+
+        def record(self):
+            pass
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, end):
+            return next(times)
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: torch.zeros(4, dtype=torch.int))
+    assert tuner_mod.JITTuner.time_candidate(lambda *a: 0, (), launches=20) == min(batches[-3:])
+    assert next(times, None) is None
+
+
 def test_tuner_fails_when_nothing_is_legal(monkeypatch, tmp_path):
     table = {"k<1>": FakeRuntime(1, rc=1), "k<2>": FakeRuntime(2, rc=1)}
     t = _fake_tuner(monkeypatch, table, tmp_path)
