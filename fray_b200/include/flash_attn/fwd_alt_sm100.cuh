@@ -643,6 +643,7 @@ attn_fwd_alt_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   }
 
+  if (*abort_flag == 1u) settle_after_abort();
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync_all();  // neither CTA leaves while the other may still signal it

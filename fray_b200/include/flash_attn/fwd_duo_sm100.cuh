@@ -570,6 +570,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   }
 
+  if (*abort_flag == 1u) settle_after_abort();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);

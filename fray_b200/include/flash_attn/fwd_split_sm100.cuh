@@ -316,6 +316,7 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   }
 
+  if (*abort_flag == 1u) settle_after_abort();
   // Merge: every CTA of the cluster adds up a share of the outputs over all partial results.
   tc_fence_before_sync();
   __syncthreads();

@@ -105,6 +105,15 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// End of a kernel whose waits may have run out: copies and products can still be under way into this CTA's shared and tensor
+// memory, which belong to somebody else as soon as it has left.  They take microseconds (a wait that a preempted device let run
+// out finds the rest of the pipeline moving again); every thread stays for about half a millisecond before the CTA's last
+// barrier.
+static constexpr long long kSettleCycles = 1000000LL;
+__device__ __noinline__ void settle_after_abort() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < kSettleCycles) __nanosleep(1000);
+}
 
 // Same contract as mbar_wait, but polls with the non-blocking test_wait instead of the suspending
 // try_wait.  A suspended waiter was measured to resume a few hundred cycles after the barrier

@@ -60,3 +60,18 @@ def test_a_wait_that_runs_out_raises_the_status_and_clearing_rearms():
     flash_attn_cute(q, q, q, o)
     torch.cuda.synchronize()
     assert flash_attn_status()[0] == 0 and o.abs().sum() > 0
+
+
+def test_a_cta_that_gave_up_stays_until_its_copies_have_landed():
+    from fray_b200.jit import build, generate
+    arg_defs = (("Src", torch.int), ("Out", torch.int), ("stream", torch.cuda.Stream))
+    epilogue = ('extern "C" EXPORT_API int fray_attn_status(int* out4, int clear) '
+                '{ return fray::read_attn_status(out4, clear != 0); }')
+    runtime = build("settle_probe", arg_defs, generate((f'"{os.path.join(HERE, "wait_probe.cuh")}"',), arg_defs,
+                                                       "fray_test::launch_settle_probe(Src, Out, stream, __return_code);", epilogue))
+    src, out = torch.zeros(2048, dtype=torch.int, device="cuda"), torch.zeros(3, dtype=torch.int, device="cuda")
+    assert runtime(src, out, torch.cuda.current_stream()) == 0
+    torch.cuda.synchronize()
+    gave_up, kilocycles, landed = out.tolist()
+    assert gave_up == 1 and landed == 1 and 1000 <= kilocycles < 10000
+    assert _status(runtime, clear=True)[0] == 0x7E1
