@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(640, 1)
 attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                     int num_heads, int num_bh, int seq_len, int causal, float scale_log2, int kv_group, float* lse, int seq_k,
-                    int blk, int n_kv, int n_pairs, int total) {
+                    int heaviest_first, int n_kv, int n_pairs, int total) {
   using Cfg = DuoCfg<D, STAGES>;
   constexpr int BN = Cfg::BN;
   extern __shared__ uint8_t smem_raw[];
@@ -211,24 +211,20 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
 
   const int stride = static_cast<int>(gridDim.x);
-  // Items are numbered in blocks of `blk` slices; inside a block the pairs of all its slices come heaviest first (pair by
-  // pair, slice by slice).  blk = 1 is plain slice order: CTAs that run side by side share a slice's K and V in L2.  A
-  // causal problem of few, unequal items takes blk = all slices (heaviest_first_order has the measurements).  CTA c takes
-  // the positions c, G + c, 2G + c, ...; with a causal mask the direction alternates from round to round, which evens
-  // out most of what is left.
+  // Items are numbered slice by slice (CTAs that run side by side share a slice's K and V in L2) or, with a causal mask and
+  // by duo_heaviest_first, pair by pair, the heaviest of all slices first.  CTA c takes the positions c, G + c, 2G + c, ...;
+  // with a causal mask the direction alternates from round to round, which evens out most of what is left.
   auto pos = [&](int k) {
     const int c = static_cast<int>(blockIdx.x);
     return k * stride + ((causal && (k & 1)) ? stride - 1 - c : c);  // >= total: the CTA is done; grows with k
   };
   auto decode = [&](int idx) {
     DuoItem it;
-    const int blk_items = blk * n_pairs;
-    const int blk_i = idx / blk_items;
-    const int rem = idx - blk_i * blk_items;
-    const int left = num_bh - blk_i * blk;
-    const int ns = left < blk ? left : blk;
-    const int pr = rem / ns;
-    const int bh = blk_i * blk + (rem - pr * ns);
+    const int run = heaviest_first ? num_bh : n_pairs;
+    const int hi = idx / run;
+    const int lo = idx - hi * run;
+    const int bh = heaviest_first ? lo : hi;
+    const int pr = heaviest_first ? hi : lo;
     const int pair = causal ? (n_pairs - 1 - pr) : pr;
     it.m0 = pair * (2 * Cfg::BM);
     it.b = bh / num_heads;
@@ -576,6 +572,21 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
 }
 
+// Item order of a causal problem.  The deal is fixed, so slice by slice the busiest CTA has 6 to 60 % more than its share, and
+// heaviest first evens that out; but it has all slices under way at once, and once their K and V outgrow L2 (126 MB) every item
+// fetches them from HBM, at the price of clock under the board's power limit.  Heaviest first : slice by slice, us, each
+// behind 120 ms of its own load (a first version of this comparison, the two in turn, had them share one clock and showed
+// heaviest first ahead throughout): 1 x 32 heads on 8 x 3000 x 128 (12 MB) 88 : 109 (the one-tile kernel 100), 2 x 32 on 8 x
+// 3000 163 : 175, 4 x 16 x 2048 (67 MB) 86 : 90, 1 x 16 x 8192 (67 MB) 274 : 350, 3 x 16 x 4096 (101 MB) 227 : 247, 64-wide
+// heads 2 x 32 x 3000 (49 MB) 123 : 131; 1 % behind at worst.  From 134 MB on: 4 x 32 x 2048 177 : 170, 3 x 32 x 3000 (147
+// MB) 278 : 259, 4 x 32 x 4096 (268 MB) 645 : 580, 8 x 32 on 8 x 4096 (134 MB) 1135 : 1095; with few long slices still ahead
+// a little further: 1 x 16 x 16384 (134 MB) 1030 : 1110, 1 x 32 x 8192 (134 MB) 545 : 555, but 1 x 32 x 16384 (268 MB) 2117 :
+// 2085.  Up to 1024 rows a slice's few items run side by side anyway: 2 % behind to 2 % ahead in most of 16 shapes.
+inline bool duo_heaviest_first(bool causal, const AttnShape& shp, const AttnShape& shp_kv) {
+  const long long kv_bytes = 2LL * shp_kv.B * shp_kv.H * shp_kv.S * shp_kv.D * 2;
+  return causal && shp.S > 1024 && kv_bytes <= (shp.S >= 8192 ? kHeaviestFirstMaxKvBytes : 126LL * 1000 * 1000);
+}
+
 // Host launcher for the kernel with two softmax threads per row. Returns an AttnReturnCode.
 template <int D, int STAGES>
 inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const operand_t* v, operand_t* o, const AttnShape& shp,
@@ -601,11 +612,9 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
   const int n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
   const int items = n_pairs * shp.B * shp.H;
   const int grid = items < sms ? items : sms;
-  // item order (see the kernel): heaviest first over all slices or slice by slice
-  const int blk = heaviest_first_order(causal, shp, shp_kv) ? shp.B * shp.H : 1;
   return launch_overlapped(kernel, dim3(grid), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, tm_o, shp.H,
                            shp.B * shp.H, shp.S, causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse,
-                           ex.seq_k, blk, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
+                           ex.seq_k, duo_heaviest_first(causal, shp, shp_kv) ? 1 : 0, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
 }
 
 }  // namespace sm100
