@@ -172,7 +172,8 @@ def tuning_space(d: int) -> Tuple[Dict[str, Any], ...]:
 
 
 def _forced_point() -> Optional[Dict[str, int]]:
-    forced = os.getenv("FRAY_ATTN_FORCE")  # e.g. "KIND=0,BLOCK_N=64,STAGES=1"
+    # e.g. "KIND=0,BLOCK_N=64,STAGES=1"; for bring-up: looked at when a layout is first launched, not on warm calls
+    forced = os.getenv("FRAY_ATTN_FORCE")
     if not forced:
         return None
     point = {"BLOCK_N": 128, "STAGES": 4}

@@ -6,6 +6,7 @@ Tolerances are the ones the path is specified with: max|out - torch fp16 attenti
 calc_diff(out, fp32 attention) <= 1e-5.
 """
 import ctypes
+import importlib
 import math
 import os
 
@@ -53,6 +54,8 @@ def variant(request, monkeypatch):
     else:
         monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
     _current_variant = request.param
+    # a layout launched before goes straight to the kernel it was tuned to: the variant has to be seen anew
+    importlib.import_module("fray_b200.jit_kernels.flashattn_cute")._fast_path.clear()
     yield request.param
     _current_variant = "tuned"
 

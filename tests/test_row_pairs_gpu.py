@@ -21,6 +21,7 @@ def test_row_pairs(B, H, Hkv, Sq, Sk, causal, D, gain, monkeypatch):
     monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
     point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
     monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    op._fast_path.clear()  # a layout launched before would go straight to the kernel it was tuned to
     g = torch.Generator(device="cuda").manual_seed(81)
     q = (gain * torch.randn(B, H, Sq, D, generator=g, device="cuda")).half()  # gain 6: offsets move during a row
     k, v = (torch.randn(B, Hkv, Sk, D, generator=g, device="cuda").half() for _ in range(2))
@@ -56,6 +57,7 @@ def test_finished_tiles_follow_each_other_closely(B, H, Hkv, Sq, Sk, causal, D, 
     monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
     point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
     monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    op._fast_path.clear()  # a layout launched before would go straight to the kernel it was tuned to
     g = torch.Generator(device="cuda").manual_seed(83)
     q = torch.randn(B, H, Sq, D, generator=g, device="cuda").to(dtype)
     k, v = (torch.randn(B, Hkv, Sk, D, generator=g, device="cuda").to(dtype) for _ in range(2))
@@ -89,6 +91,7 @@ def test_halves_of_a_row_agree_in_items_of_one_step(Sq, Sk, D, monkeypatch):
     monkeypatch.delenv("FRAY_ATTN_FORCE", raising=False)
     point = next(p for p in op.tuning_space(D) if p["KIND"] == op.KIND_ROW_PAIRS)
     monkeypatch.setenv("FRAY_ATTN_FORCE", ",".join(f"{k}={v}" for k, v in point.items()))
+    op._fast_path.clear()  # a layout launched before would go straight to the kernel it was tuned to
     g = torch.Generator(device="cuda").manual_seed(89)
     B, H = 4, 150
     q = (6.0 * torch.randn(B, H, Sq, D, generator=g, device="cuda")).half()
