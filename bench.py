@@ -35,11 +35,12 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 NOMINAL_FP16_TFLOPS = 2250.0
-# DRAM traffic of the warp-specialised two-tile kernel from the ncu capture summarised in
-# profiles/attn_fwd_ws_small_ncu.md (32 (b,h) units of S=4096, D=128, non-causal):
-# dram__bytes_read.sum + dram__bytes_write.sum.  Units are independent, so a launch with more units of
-# the same shape moves proportionally more.
-NCU_DRAM_BYTES_PER_UNIT_S4096_D128 = (100.783360e6 + 14.093824e6) / 32
+# DRAM traffic of the kernel with two softmax threads per row from the ncu captures summarised in
+# profiles/attn_fwd_duo_small_ncu.md (32 (b,h) units of S=4096, D=128, non-causal): dram__bytes_read.sum of a
+# launch on a flushed L2, dram__bytes_write.sum of a launch behind others of its kind (a single launch leaves
+# most of its output in L2).  Units are independent, so a launch with more units of the same shape moves
+# proportionally more.
+NCU_DRAM_BYTES_PER_UNIT_S4096_D128 = (100.742656e6 + 33.277184e6) / 32
 FALLBACK_PEAKS = {"bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "hbm_gbs": 6650.0}
 
 WORKLOADS = {
@@ -446,8 +447,8 @@ def main():
             "verify": verdict,
             "roofline": {"bound": "tensor", "achieved": per_gpu, "peak": peak, "unit": "TFLOP/s",
                          "frac": per_gpu / peak, "traffic": traffic,
-                         "traffic_note": "bytes per launch per GPU: ncu capture of the one-batch case "
-                                         "(profiles/attn_fwd_ws_small_ncu.md) scaled by the units launched",
+                         "traffic_note": "bytes per launch per GPU: ncu captures of the one-batch case "
+                                         "(profiles/attn_fwd_duo_small_ncu.md) scaled by the units launched",
                          "algorithmic_bytes": 4 * n_local * S * D * 2,
                          "peak_source": f"{peak_src} burst bf16 GEMM (MEASURED_PEAKS.json bf16_tflops)",
                          "frac_of_nominal_2250": per_gpu / NOMINAL_FP16_TFLOPS,

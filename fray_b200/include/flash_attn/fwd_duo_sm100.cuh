@@ -28,11 +28,11 @@
 //   * Values a step does not need are worked out again per item instead of kept: 104 registers hold a half row and its
 //     P without spills (10 % against the first version, which spilled 100 bytes).
 //
-// Measured against the one-thread kernels, at the clock the board keeps under load (us, same run): 4 x 32 x 4096 x 128
-// 955-998 : 1072-1108, causal 545-570 : 701-717, 1 x 32 x 16384 causal 1997-2022 : 2258-2306, 2 x 16 x 2048 70-76 : 73-75
-// (two tiles per CTA); 16 x 16 x 1024 x 64 103 : 120 (that kernel's persistent form, which this one replaces);
-// 16 x 16 x 1024 x 128 causal 95 : 121, 8 x 16 x 4096 x 64 690 : 855, 4 x 16 x 2048 x 64 causal 66 : 83 (one tile).  3400 cycles per 128 keys of two tiles, tensor pipe
-// active 60 % of a full SM's time, issue slots 43 %.  Tried and left out: 12 or 25 % of the exponentials as a degree-5
+// Measured against the faster of the two-tile and the one-tile kernel, each behind 150 ms of its own load (us, same run): 4 x
+// 32 x 4096 x 128 981-1028 : 1051-1099, causal 569-572 : 648-656, 1 x 32 x 16384 causal 2070-2080 : 2180-2261, 2 x 16 x 2048 75 :
+// 79, 16 x 16 x 1024 x 64 103 : 122, 16 x 16 x 1024 x 128 causal 105 : 127, 8 x 16 x 4096 x 64 721-726 : 801-807, 4 x 16 x 2048
+// x 64 causal 59 : 83; 20 launches of the first from an idle board 853-890 : 909-956.  3200 cycles per 128 keys of two tiles,
+// tensor pipe active 64 % of a full SM's time, issue slots 41 %.  Tried and left out: 12 or 25 % of the exponentials as a degree-5
 // polynomial on the FMA pipe (-8 %: it lengthens the chain, the special-function unit is not what limits), polling instead
 // of suspending waits in the MMA warp or the softmax warps (level), 6 or 8 ring slots at head dim 64
 // (level), at head dim 64 a P buffer of its own, which breaks the chain but adds two barriers per step (716 : 690 us at

@@ -19,8 +19,9 @@
 //     tensor pipe never waits for a softmax of its own step.
 //
 // Measured (device time, back to back on three sets of buffers): 8 x 8 K/V heads x 8192 keys x 128 bf16, 4 query heads
-// each 43.6 us = 6.2 TB/s (one 128-row tile per query head: 124 us); 1 x 8 x 16384 18.7 us (206 us); 16 x 8 x 16384 with
-// 8 query heads each 160 us (1020 us); 2 x 8 heads x 100 queries x 2000 keys 14.5 us (31 us).
+// each 44.4-45.3 us = 6.0 TB/s (one 128-row tile per query head in the two-tile kernel: 142 us); 1 x 8 x 16384 17.5 us (197
+// us); 16 x 8 x 16384 with 8 query heads each 162-174 us (1377 us); 2 x 8 heads x 100 queries x 2000 keys 13.1 us (29 us,
+// alternating kernel 21 us).
 //
 // Warps 0-3 softmax and epilogue, warp 4 MMA issue, warp 5 TMA producer, warps 6-7 help with the merge.
 // Every barrier wait is bounded (see sm100_ptx.cuh).
