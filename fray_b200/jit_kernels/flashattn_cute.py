@@ -162,10 +162,35 @@ def _split_keys(slices: int, seq_len: int, seq_len_kv: int, causal: bool, sms: i
     return steps >= (8 if d == 64 or 12 * items <= sms else 12)
 
 
-def _folds(t: torch.Tensor) -> bool:
+# Sizes and element strides cross the C ABI as 32-bit integers, which ctypes fills without a check.
+_ABI_INT_MAX = 2 ** 31 - 1
+
+
+def _folds(t: torch.Tensor, num_kv_heads: int = 1) -> bool:
     """Whether the heads of ``t`` follow each other as further rows do: the query heads of a K/V head's group are then one
-    longer sequence of queries to it (without a causal mask, where a query's place in its head counts)."""
-    return t.stride(1) == t.shape[2] * t.stride(2)
+    longer sequence of queries to it (without a causal mask, where a query's place in its head counts), as long as its length,
+    rounded up to whole tiles, and the step from group to group still fit the ABI."""
+    group = t.shape[1] // num_kv_heads
+    return (t.stride(1) == t.shape[2] * t.stride(2) and group * t.shape[2] <= _ABI_INT_MAX - 255
+            and (num_kv_heads == 1 or group * t.stride(1) <= _ABI_INT_MAX))
+
+
+def _launch_args(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, may_fold: bool) -> tuple:
+    """The arguments of ``launch`` that the operands fix: ``(q, k, v, out, batch, heads, queries, 12 strides, K/V heads, keys)``.
+
+    With ``may_fold`` there is one slice per K/V head instead of per query head where the layout allows it: fewer tiles that end
+    early, and K and V are fetched once for rows that share a tile.  2 x 16/4 x 513 on 6000 x 128: 12 times 256 rows per K/V
+    head become 9.
+    """
+    batch_size, num_heads, seq_len, d = q.shape
+    num_kv_heads, seq_len_kv = k.shape[1], k.shape[2]
+    group = num_heads // num_kv_heads
+    if may_fold and group > 1 and seq_len > 1 and _folds(q, num_kv_heads) and _folds(out, num_kv_heads):
+        num_heads, seq_len = num_kv_heads, group * seq_len
+        q, out = (t.as_strided((batch_size, num_heads, seq_len, d), (t.stride(0), group * t.stride(1), t.stride(2), 1))
+                  for t in (q, out))
+    strides = tuple(int(t.stride(i)) if t.shape[i] > 1 else 8 for t in (q, k, v, out) for i in range(3))
+    return (q, k, v, out, int(batch_size), int(num_heads), int(seq_len), *strides, int(num_kv_heads), int(seq_len_kv))
 
 
 def tuning_space(d: int) -> Tuple[Dict[str, Any], ...]:
@@ -362,12 +387,6 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
     forced = os.getenv("FRAY_ATTN_FORCE", "")
     few = not forced and _few_queries(num_heads // num_kv_heads, seq_len, seq_len_kv, bool(causal), batch_size * num_kv_heads,
                                       sms, d)
-    # One slice per K/V head instead of per query head: fewer tiles that end early, and K and V are fetched once for rows that
-    # share a tile.  2 x 16/4 x 513 on 6000 x 128: 12 times 256 rows per K/V head become 9.
-    group = num_heads // num_kv_heads
-    fold = group > 1 and seq_len > 1 and not causal and not few and _folds(q) and _folds(out)
-    if fold:
-        num_heads, seq_len = num_kv_heads, group * seq_len
     stream = torch.cuda.current_stream(Q.device)
     sm_scale = float(scale) if scale is not None else 1.0 / math.sqrt(d)
     assert sm_scale > 0 and math.isfinite(sm_scale), "the softmax scale must be positive and finite"
@@ -379,14 +398,10 @@ def flash_attn_cute(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Output: t
             lse_arg = _no_lse[Q.device] = torch.empty(0, dtype=torch.float32, device=Q.device)
 
     def pack(q, k, v, out):
-        if fold:
-            q, out = (t.as_strided((batch_size, num_heads, seq_len, d), (t.stride(0), group * t.stride(1), t.stride(2), 1))
-                      for t in (q, out))
-        strides = tuple(int(t.stride(i)) if t.shape[i] > 1 else 8 for t in (q, k, v, out) for i in range(3))
-        return (q, k, v, out, int(batch_size), int(num_heads), int(seq_len), *strides, int(num_kv_heads),
-                int(seq_len_kv), lse_arg, bool(causal), sm_scale, stream)
+        return (*_launch_args(q, k, v, out, may_fold=not causal and not few), lse_arg, bool(causal), sm_scale, stream)
 
     args = pack(q, k, v, out)
+    num_heads, seq_len = args[5:7]
     split = not forced and not few and _split_keys(batch_size * num_heads, seq_len, seq_len_kv, bool(causal), sms, d)
     runtime = jit_tuner.compile_and_tune(
         name="flash_attn_cute",
