@@ -190,6 +190,9 @@ def _launch_args(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.T
         q, out = (t.as_strided((batch_size, num_heads, seq_len, d), (t.stride(0), group * t.stride(1), t.stride(2), 1))
                   for t in (q, out))
     strides = tuple(int(t.stride(i)) if t.shape[i] > 1 else 8 for t in (q, k, v, out) for i in range(3))
+    if max(*strides, seq_len, seq_len_kv) > _ABI_INT_MAX:
+        raise RuntimeError(f"flash_attn_cute: sizes and strides are limited to {_ABI_INT_MAX} elements (strides {strides}, "
+                           f"{seq_len} queries, {seq_len_kv} keys)")
     return (q, k, v, out, int(batch_size), int(num_heads), int(seq_len), *strides, int(num_kv_heads), int(seq_len_kv))
 
 

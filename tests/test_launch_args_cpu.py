@@ -1,4 +1,4 @@
-"""Folded groups of query heads reach `launch` with strides that fit: the ABI has 32 bits for each, and ctypes wraps silently.
+"""Sizes and strides reach `launch` as they are, or the call is refused: the ABI has 32 bits for each, and ctypes wraps silently.
 Tensors of the sizes that matter have no storage here, and the kernel library is faked."""
 import importlib
 import types
@@ -75,3 +75,21 @@ def test_folded_length_leaves_room_for_whole_tiles(launched, rows):
     call(1, 8, 1, rows, 64, view=overlapping)
     heads, n, _, _ = sizes(launched[0])
     assert (heads, n) == ((1, 8 * rows) if 8 * rows + 255 < 2 ** 31 else (8, rows))
+
+
+# contiguous tensors are handed on as they are, whatever their strides: these wrap to 8 * n, to 0 and to a negative number
+@pytest.mark.parametrize("H,S", [(8, 2 ** 22 + 8), (8, 2 ** 22), (8, 2 ** 21)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_contiguous_strides_that_do_not_fit_are_refused(launched, H, S, causal):
+    with pytest.raises(RuntimeError):
+        call(2, H, H, S, 128, causal=causal)
+    with pytest.raises(RuntimeError):
+        call(2, H, H, 64, 128, Sk=S, causal=causal)
+    assert not launched
+
+
+def test_strides_that_fit_are_not_refused(launched):
+    call(2, 8, 8, 2 ** 21 - 8, 128, causal=True)
+    assert launched[0][7] == 8 * (2 ** 21 - 8) * 128
+    call(1, 8, 8, 2 ** 22, 128)  # the batch stride of one batch is not stepped over
+    assert sizes(launched[1])[2][1:] == (2 ** 29, 128)
