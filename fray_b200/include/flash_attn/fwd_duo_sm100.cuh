@@ -806,6 +806,44 @@ inline int duo_parts(int items, int steps, bool causal, int sms, const int (&act
   return best;
 }
 
+// Whether it can be more than one, as a test that asks the device nothing: two CTAs per item have to fit, and up to four steps even
+// the best split costs what it saves (a step each and the merge: 7, against 4 + 3).  The smallest calls run at the host's pace, and
+// what duo_parts needs from the device costs it 0.1 to 0.2 us a call (4 heads of 256 rows: 6.20 -> 6.00 us).
+inline bool duo_may_split(int items, int steps, int sms) { return 2 * items <= sms && steps > 4; }
+
+// How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit).
+struct DuoPlan {
+  DuoMode mode;
+  int parts, sms, items, n_pairs, n_kv;
+};
+
+template <int D, int STAGES>
+inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, cudaStream_t stream, DuoPlan& plan) {
+  using Cfg = DuoCfg<D, STAGES>;
+  plan.mode = kDuoDealt;
+  plan.parts = 1;
+  plan.sms = device_sm_count();
+  if (plan.sms <= 0) return kAttnLaunchFailed;
+  plan.n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
+  plan.n_kv = (shp_kv.S + Cfg::BN - 1) / Cfg::BN;
+  plan.items = plan.n_pairs * shp.B * shp.H;
+  const int steps = causal && 2 * plan.n_pairs < plan.n_kv ? 2 * plan.n_pairs : plan.n_kv;
+  if (duo_may_split(plan.items, steps, plan.sms)) {
+    auto split = attn_fwd_duo_kernel<D, STAGES, kDuoSplit>;
+    struct Tag {};
+    const int rc = ensure_dynamic_smem<Tag>(split, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
+    if (rc != kAttnOk) return rc;
+    ClusterLaunch launch(plan.items, Cfg::kThreads, Cfg::kSmemBytes, stream);
+    const auto* active = active_cluster_counts<Tag>(split, launch);
+    if (active == nullptr) return kAttnLaunchFailed;
+    plan.parts = duo_parts(plan.items, steps, causal, plan.sms, *active);
+    if (plan.parts > 1) plan.mode = kDuoSplit;
+  } else if (duo_matched(causal, shp, shp_kv, plan.n_pairs, plan.sms, Cfg::kMaxDeal)) {  // two items per SM and more
+    plan.mode = kDuoMatched;
+  }
+  return kAttnOk;
+}
+
 // Host launcher for the kernel with two softmax threads per row. Returns an AttnReturnCode.
 template <int D, int STAGES>
 inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const operand_t* v, operand_t* o, const AttnShape& shp,
@@ -823,41 +861,29 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
   rc = cached_attn_tensor_map(&tm_o, o, shp, st[3], Cfg::BM);
   if (rc != kAttnOk) return rc;
 
-  auto kernel = attn_fwd_duo_kernel<D, STAGES, kDuoDealt>;
-  rc = ensure_dynamic_smem<Cfg>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
+  DuoPlan plan;
+  rc = duo_plan<D, STAGES>(shp, shp_kv, causal, stream, plan);
   if (rc != kAttnOk) return rc;
-  const int sms = device_sm_count();
-  if (sms <= 0) return kAttnLaunchFailed;
-  const int n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
-  const int items = n_pairs * shp.B * shp.H;
-  const int grid = items < sms ? items : sms;
-  const int n_kv = (ex.seq_k + Cfg::BN - 1) / Cfg::BN;
-  if (2 * items <= sms) {
-    auto split = attn_fwd_duo_kernel<D, STAGES, kDuoSplit>;
-    struct Tag {};
-    rc = ensure_dynamic_smem<Tag>(split, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
-    if (rc != kAttnOk) return rc;
-    ClusterLaunch launch(items, Cfg::kThreads, Cfg::kSmemBytes, stream);
-    const auto* active = active_cluster_counts<Tag>(split, launch);
-    if (active == nullptr) return kAttnLaunchFailed;
-    const int parts = duo_parts(items, causal && 2 * n_pairs < n_kv ? 2 * n_pairs : n_kv, causal, sms, *active);
-    if (parts > 1) {
-      launch.set_ctas(parts);
-      const DuoOut out{o, shp.B > 1 ? st[3].b : 0, shp.H > 1 ? st[3].h : 0, shp.S > 1 ? st[3].s : 0};
-      return launch(split, tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0, scale * 1.44269504088896340736f,
-                    ex.kv_group, ex.lse, ex.seq_k, 1, n_kv, n_pairs, items, parts, out);
-    }
+  const float scale_log2 = scale * 1.44269504088896340736f;
+  if (plan.mode == kDuoSplit) {
+    ClusterLaunch launch(plan.items, Cfg::kThreads, Cfg::kSmemBytes, stream);
+    launch.set_ctas(plan.parts);
+    const DuoOut out{o, shp.B > 1 ? st[3].b : 0, shp.H > 1 ? st[3].h : 0, shp.S > 1 ? st[3].s : 0};
+    return launch(attn_fwd_duo_kernel<D, STAGES, kDuoSplit>, tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0,
+                  scale_log2, ex.kv_group, ex.lse, ex.seq_k, 1, plan.n_kv, plan.n_pairs, plan.items, plan.parts, out);
   }
-  if (duo_matched(causal, shp, shp_kv, n_pairs, sms, Cfg::kMaxDeal)) {
+  auto kernel = attn_fwd_duo_kernel<D, STAGES, kDuoDealt>;
+  if (plan.mode == kDuoMatched) {
     struct Tag {};
-    auto matched = attn_fwd_duo_kernel<D, STAGES, kDuoMatched>;
-    rc = ensure_dynamic_smem<Tag>(matched, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
-    if (rc != kAttnOk) return rc;
-    kernel = matched;
+    kernel = attn_fwd_duo_kernel<D, STAGES, kDuoMatched>;
+    rc = ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
+  } else {
+    rc = ensure_dynamic_smem<Cfg>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
   }
-  return launch_overlapped(kernel, dim3(grid), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q, tm_k, tm_v, tm_o, shp.H,
-                           shp.B * shp.H, shp.S, causal ? 1 : 0, scale * 1.44269504088896340736f, ex.kv_group, ex.lse,
-                           ex.seq_k, duo_heaviest_first(causal, shp, shp_kv) ? 1 : 0, n_kv, n_pairs, items, 1, DuoOut{});
+  if (rc != kAttnOk) return rc;
+  return launch_overlapped(kernel, dim3(plan.items < plan.sms ? plan.items : plan.sms), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q,
+                           tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0, scale_log2, ex.kv_group, ex.lse, ex.seq_k,
+                           duo_heaviest_first(causal, shp, shp_kv) ? 1 : 0, plan.n_kv, plan.n_pairs, plan.items, 1, DuoOut{});
 }
 
 }  // namespace sm100

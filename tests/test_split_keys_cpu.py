@@ -1,6 +1,8 @@
 """The rule that sends calls to the row-pair kernel with split keys, at its edges, and which groups of heads are folded."""
+import ctypes
 import importlib
 
+import pytest
 import torch
 
 op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
@@ -28,3 +30,49 @@ def test_calls_the_rule_leaves():
 def test_heads_that_follow_each_other_as_rows_do():
     t = torch.empty(2, 4, 10, 64)
     assert op._folds(t) and not op._folds(t[:, :, :9]) and not op._folds(torch.empty(2, 10, 4, 64).transpose(1, 2))
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    """The launcher's rules, which are host code: parts(items, steps, causal, sms, active) and may_split(items, steps, sms)."""
+    from fray_b200.jit import build, generate
+    args = (("n", int),)
+    code = generate(op.includes, args, "\n__return_code = 0;\n", """
+extern "C" EXPORT_API int parts(int items, int steps, int causal, int sms, const int* active) {
+    return fray::sm100::duo_parts(items, steps, causal != 0, sms, *reinterpret_cast<const int (*)[fray::kMaxClusterCtas + 1]>(active));
+}
+extern "C" EXPORT_API int may_split(int items, int steps, int sms) { return fray::sm100::duo_may_split(items, steps, sms); }
+""")
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setenv("FRAY_CACHE_DIR", str(tmp_path_factory.mktemp("rules")))
+        lib = build("split_rules", args, code)
+    parts, may_split = lib.symbol("parts"), lib.symbol("may_split")
+    return (lambda items, steps, causal, sms, active: parts(items, steps, causal, sms, (ctypes.c_int * 9)(*active))), may_split
+
+
+# clusters of 1 to 8 CTAs that run at the same time on 148 SMs: as many as the SMs allow at best, and as on a device whose GPCs
+# leave some over
+PLACES = [(0, 148, 74, 49, 37, 29, 24, 21, 18), (0, 148, 74, 47, 35, 27, 22, 18, 16), (0, 148, 70, 40, 30, 0, 0, 0, 0)]
+
+
+@pytest.mark.parametrize("places", PLACES)
+def test_calls_that_are_not_looked_at_would_not_be_split(rules, places):
+    parts, may_split = rules
+    for items in range(1, 200):
+        for steps in range(1, 60):
+            for causal in (0, 1):
+                n = parts(items, steps, causal, 148, places)
+                assert 1 <= n <= min(8, steps)
+                if not may_split(items, steps, 148):
+                    assert n == 1 or 2 * items > 148  # two CTAs per item do not fit
+                if causal and n > 1:
+                    assert items <= places[n]
+
+
+def test_parts_of_some_calls(rules):
+    parts, may_split = rules
+    assert not may_split(4, 2, 148) and not may_split(75, 47, 148) and may_split(74, 5, 148)
+    first = PLACES[0]
+    assert [parts(n, 47, 0, 148, first) for n in (1, 18, 37, 38, 50, 72, 74)] == [8, 8, 4, 3, 2, 2, 2]
+    assert [parts(n, 20, 0, 148, first) for n in (50, 72)] == [2, 2] and parts(64, 32, 1, 148, first) == 2
+    assert parts(71, 32, 1, 148, PLACES[2]) == 1  # causal: a second round is not looked at
