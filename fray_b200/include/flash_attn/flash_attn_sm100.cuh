@@ -95,4 +95,21 @@ inline void flash_attn_layout(void* q, void* k, void* v, void* o, void* lse, voi
       l.scale, static_cast<cudaStream_t>(stream), rc);
 }
 
+// How a launch of this layout on the current device deals its work, for tests and tools: mode (DuoMode; 0 for every other kind) and
+// CTAs per work item.  Returns an AttnReturnCode.
+template <int KIND, int D, int STAGES>
+inline int flash_attn_form(const AttnLayout& l, int* mode, int* parts) {
+  *mode = 0;
+  *parts = 1;
+  if constexpr (KIND == kAttnDuo || KIND == kAttnPersistent) {
+    sm100::DuoPlan plan;
+    const int rc = sm100::duo_plan<D, STAGES>(AttnShape{l.batch_size, l.num_heads, l.seq_len, D},
+                                              AttnShape{l.batch_size, l.num_kv_heads, l.seq_len_kv, D}, l.causal != 0, nullptr, plan);
+    if (rc != kAttnOk) return rc;
+    *mode = plan.mode;
+    *parts = plan.parts;
+  }
+  return kAttnOk;
+}
+
 }  // namespace fray

@@ -50,6 +50,9 @@ extern "C" EXPORT_API int fray_attn_launch_layout(void* Q, void* K, void* V, voi
     fray::flash_attn_layout<{KIND}, {D}, {BLOCK_N}, {STAGES}>(Q, K, V, O, Lse, stream, *l, rc);
     return rc;
 }
+extern "C" EXPORT_API int fray_attn_form(const fray::AttnLayout* l, int* mode, int* parts) {
+    return fray::flash_attn_form<{KIND}, {D}, {STAGES}>(*l, mode, parts);
+}
 #ifdef FRAY_ATTN_TRACE
 extern "C" EXPORT_API int fray_attn_trace_read(unsigned int* out, int max_words) {
     return fray::sm100::read_attn_trace(out, max_words);
