@@ -244,9 +244,13 @@ def _forced_point() -> Optional[Dict[str, int]]:
 
 def _workload_class(seq_len: int, seq_len_kv: int, units: int, sms: int) -> str:
     """Coarse workload class the tuner memoises on, from what the kinds differ in: how many steps a work item has (bucket of
-    the number of keys), whether items of two query tiles fill the chip, and whether there is a second tile at all."""
+    the number of keys), whether items of two query tiles fill the chip, and whether there is a second tile at all.  Items of
+    more than four steps for up to half of the SMs are apart: two and more CTAs can share one (row-pair kernel), or have an SM
+    each (one-tile kernels).  As one class, 256 rows a head, the call that came first decided: 48 heads 20.1 us on 2048 keys, or
+    27.5 behind 140 heads (head dim 128); 140 heads 74.3 on 6000 keys, or 86.9 behind 48 (head dim 64)."""
     k_bucket = 1 << max(7, (max(seq_len_kv, 1) - 1).bit_length())
-    fill = "big" if units * -(-seq_len // 256) >= sms else "small"
+    items = units * -(-seq_len // 256)
+    fill = "big" if items >= sms else "half" if 2 * items <= sms and seq_len_kv > 512 else "small"
     return f"K{min(k_bucket, 16384)}_{fill}{'_one_tile' if seq_len <= 128 else ''}"
 
 
