@@ -454,16 +454,17 @@ _host_staging: Dict[Any, Any] = {}
 _host_staging_lock = threading.Lock()
 
 
-# From here on the staging buffers (two slices) are kept at a quarter of the operands, as five slices' would be two thirds.
+# From here on the staging buffers (two slices) are kept at a quarter of the operands, as five slices' would be two thirds (2.5 GB).
+# Five slices against nine and eight equal ones, us: 0.5 GB of operands 8030, 8240, 8340; 1 GB 15700, 15930, 16200; 2 GB 31060,
+# 31330, 31930; 3.9 GB 59860, 60200, 61600.  Where the device has no room for them, eight equal slices.
 _LARGE_HOST_CALL_BYTES = 4 << 30
 
 
 def _slice_bounds(units: int, chunks: Optional[int], nbytes: int = 0) -> list:
     """Where the slices of a host-buffer call begin and end: ``chunks`` equal ones, or by default five that get smaller (nine for
-    large operands, ``nbytes``).  A copy
-    costs the link 3.7 us beside its bytes, so few slices; what follows the last copy-in is one slice's kernel and copy-out, so
-    the last one is small.  4 x 16 x 1024 x 128, with eight equal slices before: 1269 -> 1180 us,
-    2 x 16 x 512 594 -> 396, 4 x 32 x 4096 8420 -> 8070 (the nine: 8310).
+    large operands, ``nbytes``).  A copy costs the link 3.7 us beside its bytes, so few slices; what follows the last copy-in is
+    one slice's kernel and copy-out, so the last one is small.  4 x 16 x 1024 x 128, with eight equal slices before: 1269 -> 1180
+    us, 2 x 16 x 512 594 -> 396, 4 x 32 x 4096 8420 -> 8070 (the nine: 8310).
     """
     if chunks:
         n = max(1, min(units, chunks))
@@ -518,6 +519,7 @@ def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Outp
     Lu = lse.view(units, group, Sq) if lse is not None else None
     bounds = _slice_bounds(units, chunks, sum(t.numel() * t.element_size() for t in tensors))
     rows = max(b1 - b0 for b0, b1 in zip(bounds, bounds[1:]))
+    equal = _slice_bounds(units, chunks or 8)
     key = (dev, rows, group, Sq, Sk, D, Q.dtype, lse is not None)
     with _host_staging_lock:
         # A graph being captured gets buffers of its own (from its pool): it runs whenever it is replayed, and events of calls
@@ -525,7 +527,7 @@ def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Outp
         capturing = torch.cuda.is_current_stream_capturing()
         st = None if capturing else _host_staging.get(key)
         if st is None:
-            def make_set():
+            def make_set(rows):
                 bufs = [torch.empty((rows, group, Sq, D), dtype=Q.dtype, device=dev),
                         torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
                         torch.empty((rows, 1, Sk, D), dtype=Q.dtype, device=dev),
@@ -535,11 +537,21 @@ def flash_attn_cute_host(Q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, Outp
                 return bufs
             if not capturing:
                 _drop_host_staging()  # one shape at a time: the buffers are as large as the operands' slices
-            st = {"bufs": [make_set(), make_set()], "s_in": torch.cuda.Stream(device=dev), "s_out": torch.cuda.Stream(device=dev),
+            fewer = -(-units // (len(equal) - 1))
+            for n in (rows, fewer):  # a device that is nearly full may have room for slices that are equal, and smaller
+                try:
+                    bufs = [make_set(n) for _ in range(2)]
+                    break
+                except torch.OutOfMemoryError:
+                    if n <= fewer:
+                        raise
+            st = {"bufs": bufs, "s_in": torch.cuda.Stream(device=dev), "s_out": torch.cuda.Stream(device=dev),
                   "computed": [None, None],   # per buffer set: kernel of the slice that last used it has finished
                   "drained": [None, None]}    # ... and its result has left the device
             if not capturing:
                 _host_staging[key] = st
+        if st["bufs"][0][0].shape[0] < rows:
+            bounds = equal
         s_in, s_out = st["s_in"], st["s_out"]
         # Kept from call to call: a call on another stream finds the sets still in use by the one before it.
         computed, drained = st["computed"], st["drained"]
