@@ -187,17 +187,6 @@ struct DuoOut {
   long long sb, sh, ss;
 };
 
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-
 // SPLIT, for problems of few items: a cluster of `parts` CTAs (blockIdx.x = item * parts + part) shares the KV tiles of one
 // item and merges the partial results (fp32, 512 bytes a row and part) through each other's shared memory: no workspace, no
 // second launch, no order between clusters.  One CTA per item left most of the chip idle, and its chain of steps set the time
