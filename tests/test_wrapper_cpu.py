@@ -69,8 +69,8 @@ def test_workload_classes_tell_query_tiles_from_keys():
     assert len({chunk, square, decode, cross}) == 4
     assert cls(6000, 6000, 32, 148) == cls(8192, 8192, 32, 148) == cls(5000, 4097, 128, 148)   # a bucket is a power of two of keys
     assert cls(256, 4096, 148, 148) != cls(256, 4096, 147, 148)                                # items of 256 rows against the SMs
-    assert cls(256, 4096, 74, 148) != cls(256, 4096, 75, 148)                                  # two CTAs per item fit or do not
-    assert cls(256, 512, 74, 148) == cls(256, 512, 75, 148)                                    # four steps: nothing to split
+    # two CTAs per item fit or do not, and an SM for each 128-row tile
+    assert cls(256, 4096, 74, 148) != cls(256, 4096, 75, 148) and cls(333, 333, 37, 148) != cls(333, 333, 38, 148)
     assert cls(128, 4096, 500, 148) != cls(129, 4096, 500, 148)                                # a second query tile or none
     assert cls(40000, 40000, 32, 148) == cls(16384, 16384, 32, 148) and cls(1, 1, 1, 148) == cls(64, 128, 1, 148)
 
