@@ -32,9 +32,10 @@
 // 32 x 4096 x 128 981-1028 : 1051-1099, causal 569-572 : 648-656, 1 x 32 x 16384 causal 2070-2080 : 2180-2261, 2 x 16 x 2048 75 :
 // 79, 16 x 16 x 1024 x 64 103 : 122, 16 x 16 x 1024 x 128 causal 105 : 127, 8 x 16 x 4096 x 64 721-726 : 801-807, 4 x 16 x 2048
 // x 64 causal 59 : 83; 20 launches of the first from an idle board 853-890 : 909-956 (with products issued as they are now:
-// 823-840, see the MMA warp).  2870 cycles per 128 keys of two tiles.  Tried and left out: 12 or 25 % of the exponentials as a degree-5
-// polynomial on the FMA pipe (-8 %: it lengthens the chain, the special-function unit is not what limits), polling instead
-// of suspending waits in the MMA warp or the softmax warps (level), 6 or 8 ring slots at head dim 64
+// 823-840, see the MMA warp).  2870 cycles per 128 keys of two tiles inside an item; an item costs 2 to 3 us beside its steps.
+// Tried and left out while products were still issued instruction by instruction, which kept the MMA warp busy for a tile's whole
+// step (so these show what lost then, not that it loses now): 12 or 25 % of the exponentials as a degree-5 polynomial on the FMA
+// pipe (-8 %), polling instead of suspending waits in the MMA warp or the softmax warps (level), 6 or 8 ring slots at head dim 64
 // (level), at head dim 64 a P buffer of its own, which breaks the chain but adds two barriers per step (716 : 690 us at
 // 8 x 16 x 4096), the second fetch of scores issued ahead of the first exponentials (-2 %).
 //
@@ -69,7 +70,9 @@ struct DuoCfg {
   static constexpr int kNumBars = 2 * 2 + 2 * STAGES + 2 * 3 + 2 * kPChunks + 3;
   static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // [2 tiles][2 halves][128]
   static constexpr int kOffDeal = kOffStats + 4 * 128 * 4;
-  static constexpr int kMaxDeal = 190;  // kDuoMatched: a CTA's items and the end mark
+  // kDuoMatched: a CTA's items and the end mark, as many as shared memory has room for at head dim 128 and four slots: 189 items
+  // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
+  static constexpr int kMaxDeal = 190;
   static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
   // slack to bring the dynamic segment to a 1024-byte boundary (its base is one already; the kernel checks)
   static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
