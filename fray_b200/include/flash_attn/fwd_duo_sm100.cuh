@@ -42,6 +42,8 @@
 // Every barrier wait is bounded (see sm100_ptx.cuh), and what a warp does next never depends on whether a wait ran out, so
 // the named barriers always meet: a protocol error ends as a status word and a wrong answer, never as a hung GPU.
 
+#include <type_traits>
+
 #include "host_sm100.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_tile_sm100.cuh"
@@ -74,8 +76,7 @@ struct DuoCfg {
   // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
   static constexpr int kMaxDeal = 190;
   static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
-  // slack to bring the dynamic segment to a 1024-byte boundary (its base is one already; the kernel checks)
-  static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
+  static constexpr int kSmemBytes = kUsedBytes;
   static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
   static constexpr int kPartStride = D + 4;  // SPLIT: floats from row to row of the partial results
   static constexpr int kOffPartMl = 2 * BM * kPartStride * 4;
@@ -87,6 +88,12 @@ struct DuoCfg {
   static constexpr int kRegsTotal = 512 * kRegsSoftmax + 128 * kRegsOther;
   static_assert(kRegsTotal <= kThreads * kRegsLaunch, "register budgets exceed the CTA's allocation");
 };
+
+// Arrives on a barrier, by pointer or by its shared-memory address.
+__device__ __forceinline__ void arrive_on(uint64_t* bar) { mbar_arrive(bar); }
+__device__ __forceinline__ void arrive_on(uint32_t bar_addr) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+}
 
 // Meets the barrier and returns whether any of its threads passed `p`.
 __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
@@ -105,12 +112,14 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
 }
 
 // One step of half a row: 64 scores at t_s, the P chunks of 32 keys overwrite their head.
+// p_bar: the first chunk's barrier, by pointer or by its shared-memory address.
 // my_max: this thread's slot for the exchange of maxima, the other half's is other_off floats away; pair_bar: the named
 // barrier of the two warps that share the rows; lim (MASK): keys from lim on are past the end or above the diagonal.
-template <bool MASK, class Rescale>
-__device__ __forceinline__ void softmax_half(uint32_t t_s, uint64_t* p_bar, float* my_max, int other_off, int pair_bar,
+template <bool MASK, class Bar, class Rescale>
+__device__ __forceinline__ void softmax_half(uint32_t t_s, Bar p_bar, float* my_max, int other_off, int pair_bar,
                                              Rescale&& rescale_o, int lim, float scale_log2, int lane,
                                              float& m_ref, float& l_run) {
+  constexpr int kBarStep = std::is_pointer<Bar>::value ? 1 : 8;  // from a barrier to the next
   uint32_t sa[32], sb[32];
   tmem_ld_x32(t_s, sa);
   tmem_ld_x32(t_s + 32, sb);
@@ -151,7 +160,7 @@ __device__ __forceinline__ void softmax_half(uint32_t t_s, uint64_t* p_bar, floa
     tmem_wait_st();
     tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(p_bar + q);
+    if (lane == 0) arrive_on(p_bar + q * kBarStep);
   };
   uint32_t pk[16];
   exp_32(sa, scale2, neg_m2, rsp0, rsp1, pk);
@@ -207,10 +216,8 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   using Cfg = DuoCfg<D, STAGES>;
   constexpr int BN = Cfg::BN;
   constexpr bool SPLIT = MODE == kDuoSplit;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw_addr = smem_u32(smem_raw);
-  const uint32_t align_off = ((raw_addr + 1023u) & ~1023u) - raw_addr;
-  uint8_t* smem = smem_raw + align_off;
+  extern __shared__ __align__(1024) uint8_t duo_smem[];  // aligned by declaration: every address in it is a constant
+  uint8_t* smem = duo_smem;
   uint8_t* q_smem = smem + Cfg::kOffQ;
   uint8_t* kv_smem = smem + Cfg::kOffKV;
   uint8_t* stage_smem = smem + Cfg::kOffStage;
@@ -237,7 +244,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  if (align_off + Cfg::kUsedBytes > Cfg::kSmemBytes) {  // never seen: the segment's base is 1024-byte aligned
+  if ((smem_u32(smem) & 1023u) != 0) {  // never seen
     if (tid == 0) atomicCAS(&fray_attn_status[0], 0, 0x601);
     return;
   }
@@ -342,7 +349,15 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t t_s = tmem_base + (i == 0 ? Cfg::kColS0 : Cfg::kColS1) + hf * 64 + lane_base;
     const uint32_t t_o = tmem_base + (i == 0 ? Cfg::kColO0 : Cfg::kColO1) + hf * (D / 2) + lane_base;
-    uint64_t* p_bar = p_full + i * Cfg::kPChunks;
+    // At head dim 128 the loop's barriers go by 32-bit addresses that are worked out once; by pointers, which are converted where
+    // they are used, 1 to 3 % slower (us, behind lasting load: 4 x 32 x 4096 977 : 960, causal 548 : 534, 1 x 32 x 16384 causal
+    // 1933 : 1904).  At head dim 64 it is the other way round (8 x 16 x 4096 715 : 728, 16 x 16 x 1024 107.6 : 110).
+    auto bar_ref = [&](uint64_t* bar) {
+      if constexpr (D == 64) return bar;
+      else return smem_u32(bar);
+    };
+    const auto p_bar = bar_ref(p_full + i * Cfg::kPChunks);
+    const uint32_t s_bar = smem_u32(s_full + i);
     float* my_stat = stats + (i * 2 + hf) * 128 + r;
     const int other_off = hf ? -128 : 128;
     const int pair_bar = 1 + i * 4 + (warp & 3);
@@ -360,6 +375,10 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     };
     // phase parities, toggled: bit 0 s_full, bit 1 o_full, bit 2 stage_free
     uint32_t phases = 0;
+    auto wait_scores = [&](int j) __attribute__((always_inline)) {
+      if constexpr (D == 64) mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+      else mbar_wait(s_bar, phases & 1, abort_flag, 0x201 + i, j);
+    };
     for (int k = 0, idx = pos(0); idx < idx_end; idx = SPLIT ? idx_end : pos(++k)) {
       int n_i, n_full, lim;
       {
@@ -377,13 +396,13 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       float m_ref = -INFINITY;
       float l_run = 0.f;
       for (int j = 0; j < n_full; ++j) {
-        mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+        wait_scores(j);
         tc_fence_after_sync();
         softmax_half<false>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, 0, scale_log2, lane, m_ref, l_run);
         phases ^= 1u;
       }
       for (int j = n_full; j < n_i; ++j, lim -= BN) {
-        mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+        wait_scores(j);
         tc_fence_after_sync();
         softmax_half<true>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, lim, scale_log2, lane, m_ref, l_run);
         phases ^= 1u;
@@ -429,7 +448,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (c + 32 == D / 2) {
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(o_free + i);
+          if (lane == 0) arrive_on(bar_ref(o_free + i));
         }
         const int col = hf * (D / 2) + c;  // first column of these 32
         uint8_t* panel_row = stage_smem + (col >> 6) * Cfg::kQPanelBytes + r * 128;

@@ -64,7 +64,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar_addr, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n"
@@ -73,10 +73,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       "selp.b32 %0, 1, 0, p;\n"
       "}\n"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar_addr), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait(smem_u32(bar), parity); }
 
 __device__ __noinline__ void report_timeout(volatile uint32_t* abort_flag, uint32_t site, uint32_t extra) {
   *abort_flag = 1;
@@ -89,7 +90,9 @@ __device__ __noinline__ void report_timeout(volatile uint32_t* abort_flag, uint3
 
 // Waits for the phase with the given parity to complete. Returns early (without the
 // barrier having flipped) when the CTA abort flag is up or the cycle limit is hit.
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+// bar: the barrier, or its shared-memory address where that is known.
+template <class Bar>
+__device__ __forceinline__ void mbar_wait(Bar bar, uint32_t parity, volatile uint32_t* abort_flag,
                                           uint32_t site, uint32_t extra = 0) {
   if (mbar_try_wait(bar, parity)) return;
   const long long t0 = clock64();
