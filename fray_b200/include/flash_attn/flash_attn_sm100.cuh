@@ -112,4 +112,16 @@ inline int flash_attn_form(const AttnLayout& l, int* mode, int* parts) {
   return kAttnOk;
 }
 
+// Whether a launch of this layout on the current device puts a pair of CTAs to every work item (DuoPair), or a negative AttnReturnCode.
+template <int KIND, int D, int STAGES>
+inline int flash_attn_pair(const AttnLayout& l) {
+  if constexpr (KIND == kAttnDuo || KIND == kAttnPersistent) {
+    sm100::DuoPlan plan;
+    const int rc = sm100::duo_plan<D, STAGES>(AttnShape{l.batch_size, l.num_heads, l.seq_len, D},
+                                              AttnShape{l.batch_size, l.num_kv_heads, l.seq_len_kv, D}, l.causal != 0, nullptr, plan);
+    return rc == kAttnOk ? plan.pair : -rc;
+  }
+  return 0;
+}
+
 }  // namespace fray

@@ -9,6 +9,8 @@
 //   warp 17     TMA producer (Q tiles, K_j, V_j through a ring of STAGES buffers)
 //   warp 18     TMA stores of finished tiles
 //   warp 19     idle (fills the warpgroup for setmaxnreg)
+// At head dim 128 long calls put a pair of CTAs to an item (duo_pair): two query tiles in each of the two, every product one
+// cta_group::2 instruction that the leader's warp 16 issues for both, each CTA with half of K's rows and of V's columns.
 //
 // What bounds the kernel is the chain S(j) -> softmax -> P.V(j) -> S(j+1) of each query tile (P overwrites its S, tensor
 // memory has no room for another buffer).  With one thread per row (fwd_ws_sm100.cuh) a tile's softmax is one in-order
@@ -51,9 +53,12 @@
 namespace fray {
 namespace sm100 {
 
-template <int D, int STAGES>
+// CTAS == 2: a CTA pair works on one item, every product is one cta_group::2 instruction of 256 rows, and each CTA holds half of
+// K's rows and of V's columns.
+template <int D, int STAGES, int CTAS = 1>
 struct DuoCfg {
   static_assert(D == 64 || D == 128, "head dim must be 64 or 128");
+  static_assert(CTAS == 1 || D == 128, "a CTA of a pair holds 64 head dims of V, one 128-byte panel");
   static_assert(STAGES >= 3 && STAGES <= 8, "3..8 K/V buffers");
   static constexpr int BM = 128, BN = 128;     // rows per query tile, keys per step
   static constexpr int kThreads = 640;
@@ -65,16 +70,24 @@ struct DuoCfg {
   static constexpr int kQTileBytes = kPanels * kQPanelBytes;
   static constexpr int kKVPanelBytes = BN * 128;
   static constexpr int kKVTileBytes = kPanels * kKVPanelBytes;
+  static constexpr int kKRows = BN / CTAS;
+  static constexpr int kKPanelBytes = kKRows * 128;
+  static constexpr int kVPanels = kPanels / CTAS;
+  static constexpr int kSlotBytes = kKVTileBytes / CTAS;
+  // A pair's slots are half as large: six of them leave room for a staging tile per query tile, so that tile 1's end does not
+  // wait for tile 0's store to have been read (eight slots and one staging tile: 1.5 % more cycles on 4 x 32 x 4096).
+  static constexpr int kRing = CTAS == 2 ? 6 : STAGES;
+  static constexpr int kStageTiles = CTAS == 2 ? 2 : 1;
   static constexpr int kOffQ = 0;
   static constexpr int kOffKV = 2 * kQTileBytes;
-  static constexpr int kOffStage = kOffKV + STAGES * kKVTileBytes;  // O staging tile behind the ring, for both query tiles
-  static constexpr int kOffBars = kOffStage + kQTileBytes;
-  static constexpr int kNumBars = 2 * 2 + 2 * STAGES + 2 * 3 + 2 * kPChunks + 3;
+  static constexpr int kOffStage = kOffKV + kRing * kSlotBytes;  // O staging tile behind the ring, for both query tiles (a pair: one each)
+  static constexpr int kOffBars = kOffStage + kStageTiles * kQTileBytes;
+  static constexpr int kNumBars = 2 * 2 + 2 * kRing + 2 * 3 + 2 * kPChunks + 4;
   static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // [2 tiles][2 halves][128]
   static constexpr int kOffDeal = kOffStats + 4 * 128 * 4;
   // kDuoMatched: a CTA's items and the end mark, as many as shared memory has room for at head dim 128 and four slots: 189 items
   // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
-  static constexpr int kMaxDeal = 190;
+  static constexpr int kMaxDeal = CTAS == 2 ? 140 : 190;
   static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
   static constexpr int kSmemBytes = kUsedBytes;
   static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
@@ -89,11 +102,9 @@ struct DuoCfg {
   static_assert(kRegsTotal <= kThreads * kRegsLaunch, "register budgets exceed the CTA's allocation");
 };
 
-// Arrives on a barrier, by pointer or by its shared-memory address.
+// Arrives on a barrier: of this CTA, or by its cluster-wide address.
 __device__ __forceinline__ void arrive_on(uint64_t* bar) { mbar_arrive(bar); }
-__device__ __forceinline__ void arrive_on(uint32_t bar_addr) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
-}
+__device__ __forceinline__ void arrive_on(uint32_t cluster_addr) { mbar_arrive_cluster(cluster_addr); }
 
 // Meets the barrier and returns whether any of its threads passed `p`.
 __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
@@ -112,7 +123,7 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
 }
 
 // One step of half a row: 64 scores at t_s, the P chunks of 32 keys overwrite their head.
-// p_bar: the first chunk's barrier, by pointer or by its shared-memory address.
+// p_bar: the first chunk's barrier, by pointer or by its cluster-wide address (of a pair, the leader's).
 // my_max: this thread's slot for the exchange of maxima, the other half's is other_off floats away; pair_bar: the named
 // barrier of the two warps that share the rows; lim (MASK): keys from lim on are past the end or above the diagonal.
 template <bool MASK, class Bar, class Rescale>
@@ -187,8 +198,9 @@ __device__ __forceinline__ void softmax_half(uint32_t t_s, Bar p_bar, float* my_
 // that has as many steps less than the middle of the slice as it has more.
 enum DuoMode : int { kDuoDealt = 0, kDuoSplit = 1, kDuoMatched = 2 };
 
-// One work item: the rows [m0, m0 + 256) of slice (b, h) and the number of KV tiles each of its two query tiles consumes,
-// from tile j0 on (SPLIT; 0 otherwise).
+// One work item: two query tiles of slice (b, h) from row m0 on and the number of KV tiles each of them consumes, from tile j0 on
+// (SPLIT; 0 otherwise).  A tile is 128 rows; of a CTA pair 256 rows, 128 in each CTA, or the same 128 rows of two heads (h: this
+// CTA's) that share a K/V head.
 struct DuoItem {
   int m0, b, h, n0, n1, j0;
 };
@@ -207,31 +219,34 @@ struct DuoOut {
 // 44, 50 -> 21, 33 -> 11, 28 -> 20, 50 -> 33.  Tried and left out: equal stretches of all items' steps for any number of CTAs,
 // partial results in global memory, merged by whoever finds the others' written (9 us for the merge, and the steps 5 to 15 %
 // slower, as the items' arithmetic took registers from them).
-template <int D, int STAGES, DuoMode MODE>
+template <int D, int STAGES, DuoMode MODE, int CTAS>
 __global__ void __launch_bounds__(640, 1)
 attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                     int num_heads, int num_bh, int seq_len, int causal, float scale_log2, int kv_group, float* lse, int seq_k,
-                    int heaviest_first, int n_kv, int n_pairs, int total, int parts, const DuoOut out) {
-  using Cfg = DuoCfg<D, STAGES>;
+                    int heaviest_first, int n_kv, int n_pairs, int total, int parts, int pair_heads, const DuoOut out) {
+  using Cfg = DuoCfg<D, STAGES, CTAS>;
   constexpr int BN = Cfg::BN;
+  constexpr int RING = Cfg::kRing;
   constexpr bool SPLIT = MODE == kDuoSplit;
+  static_assert(CTAS == 1 || !SPLIT, "a split item's clusters are of single CTAs");
   extern __shared__ __align__(1024) uint8_t duo_smem[];  // aligned by declaration: every address in it is a constant
   uint8_t* smem = duo_smem;
   uint8_t* q_smem = smem + Cfg::kOffQ;
   uint8_t* kv_smem = smem + Cfg::kOffKV;
   uint8_t* stage_smem = smem + Cfg::kOffStage;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
+  // Of a pair, the barriers that both CTAs' threads or copies arrive on are the leader's (rank 0, whose warp 16 issues for both).
   uint64_t* q_full = bars;                      // [2]   producer -> MMA
   uint64_t* q_free = bars + 2;                  // [2]   MMA -> producer  (the item's last S of tile i has read Q_i)
-  uint64_t* kv_full = bars + 4;                 // [STAGES] producer -> MMA
-  uint64_t* kv_empty = kv_full + STAGES;        // [STAGES] MMA -> producer
-  uint64_t* s_full = kv_empty + STAGES;         // [2]   MMA -> softmax i
+  uint64_t* kv_full = bars + 4;                 // [RING] producer -> MMA
+  uint64_t* kv_empty = kv_full + RING;          // [RING] MMA -> producer
+  uint64_t* s_full = kv_empty + RING;           // [2]   MMA -> softmax i
   uint64_t* o_full = s_full + 2;                // [2]   MMA -> softmax i (the item's last P.V)
   uint64_t* o_free = o_full + 2;                // [2]   softmax i -> MMA (the item's O_i is in registers)
   uint64_t* p_full = o_free + 2;                // [2][kPChunks] softmax i -> MMA
-  uint64_t* stage_full = p_full + 2 * Cfg::kPChunks;  // softmax -> store warp
-  uint64_t* stage_free = stage_full + 1;        // [2]   store warp -> softmax i (the staging tile is tile i's turn)
+  uint64_t* stage_full = p_full + 2 * Cfg::kPChunks;  // [kStageTiles] softmax -> store warp
+  uint64_t* stage_free = stage_full + 2;        // [2]   store warp -> softmax i (the staging tile is tile i's turn)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::kNumBars);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
   float* stats = reinterpret_cast<float*>(smem + Cfg::kOffStats);
@@ -249,35 +264,41 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     return;
   }
 
-  const int stride = static_cast<int>(gridDim.x);
+  const int rank = CTAS == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int unit = static_cast<int>(blockIdx.x) / CTAS;
+  const int stride = static_cast<int>(gridDim.x) / CTAS;
+  // Rows from a query tile to the next, and from a tile's first row to this CTA's; heads that an item takes.
+  const int tile_rows = CTAS == 2 && !pair_heads ? 2 * Cfg::BM : Cfg::BM;
+  const int row_off = CTAS == 2 && !pair_heads ? rank * Cfg::BM : 0;
+  const int item_heads = CTAS == 2 && pair_heads ? 2 : 1;
   const int part = SPLIT ? static_cast<int>(blockIdx.x) % parts : 0;
   // Items are numbered slice by slice (CTAs that run side by side share a slice's K and V in L2) or, with a causal mask and
-  // by duo_heaviest_first, pair by pair, the heaviest of all slices first.  CTA c takes the positions c, G + c, 2G + c, ...;
+  // by duo_heaviest_first, pair by pair, the heaviest of all slices first.  CTA (CTA pair) c takes the positions c, G + c, ...;
   // with a causal mask the direction alternates from round to round, which evens out most of what is left.
   auto pos = [&](int k) {
-    const int c = static_cast<int>(blockIdx.x);
+    const int c = unit;
     if constexpr (SPLIT) return c / parts;  // its only one
     if constexpr (MODE == kDuoMatched) return static_cast<int>(deal[k]);
     return k * stride + ((causal && (k & 1)) ? stride - 1 - c : c);  // >= total: the CTA is done; grows with k
   };
   auto decode = [&](int idx) {
     DuoItem it;
-    const int run = heaviest_first ? num_bh : n_pairs;
+    const int run = heaviest_first ? num_bh / item_heads : n_pairs;
     const int hi = idx / run;
     const int lo = idx - hi * run;
     const int bh = heaviest_first ? lo : hi;
     const int pr = heaviest_first ? hi : lo;
     const int pair = causal ? (n_pairs - 1 - pr) : pr;
-    it.m0 = pair * (2 * Cfg::BM);
-    it.b = bh / num_heads;
-    it.h = bh - it.b * num_heads;
+    it.m0 = pair * (2 * tile_rows);
+    it.b = bh * item_heads / num_heads;
+    it.h = bh * item_heads - it.b * num_heads + (item_heads > 1 ? rank : 0);
     int n[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int row0 = it.m0 + i * Cfg::BM;
+      const int row0 = it.m0 + i * tile_rows;
       n[i] = row0 < seq_len ? n_kv : 0;
       if (causal && n[i] > 0) {
-        const int lim = (row0 + Cfg::BM + BN - 1) / BN;
+        const int lim = (row0 + tile_rows + BN - 1) / BN;
         n[i] = lim < n[i] ? lim : n[i];
       }
     }
@@ -298,17 +319,18 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(q_full + i, 1);
       mbar_init(q_free + i, 1);
       mbar_init(s_full + i, 1);
-      for (int c = 0; c < Cfg::kPChunks; ++c) mbar_init(p_full + i * Cfg::kPChunks + c, 8);
+      for (int c = 0; c < Cfg::kPChunks; ++c) mbar_init(p_full + i * Cfg::kPChunks + c, 8 * CTAS);
       mbar_init(o_full + i, 1);
-      mbar_init(o_free + i, 8);
+      mbar_init(o_free + i, 8 * CTAS);
     }
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < RING; ++s) {
       mbar_init(kv_full + s, 1);
       mbar_init(kv_empty + s, 1);
     }
-    mbar_init(stage_full, 8);
-    mbar_init(stage_free, 1);
-    mbar_init(stage_free + 1, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(stage_full + i, 8);
+      mbar_init(stage_free + i, 1);
+    }
     fence_barrier_init();
   }
   __syncwarp();
@@ -320,7 +342,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // Worked out once, as in the roles it took registers from the KV loop.  An odd number of pairs is matched over two slices.
     const int two = n_pairs & 1, run = n_pairs << two;
     for (int k = tid - 64; k >= 0 && k < Cfg::kMaxDeal; k += Cfg::kThreads - 64) {
-      const int d = (k >> 1) * stride + static_cast<int>(blockIdx.x);
+      const int d = (k >> 1) * stride + unit;
       const int group = 2 * d / run, j = d - group * (run >> 1), r = (k & 1) ? run - 1 - j : j;
       reinterpret_cast<uint32_t*>(smem + Cfg::kOffDeal)[k] = 2 * d < total ? ((group << two) + (r & two)) * n_pairs + (r >> two) : total;
     }
@@ -333,7 +355,14 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   // An earlier launch left the device status raised: nothing is computed (SPLIT: the cluster's barriers have to be met).
-  const bool dead = *abort_flag == 2u;
+  bool dead = *abort_flag == 2u;
+  if constexpr (CTAS == 2) {
+    // The barriers of both CTAs exist before anything arrives on them, and both agree on whether to run.
+    cluster_sync_all();
+    dead |= ld_shared_cluster_u32(mapa_shared(smem_u32(const_cast<uint32_t*>(abort_flag)), rank ^ 1)) == 2u;
+    cluster_sync_all();  // the peer has read this CTA's flag before anything may raise it
+  }
+  auto leader = [&](uint64_t* bar) { return CTAS == 2 ? mapa_shared(smem_u32(bar), 0) : smem_u32(bar); };
   if (!SPLIT && dead) {
     if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
     return;
@@ -351,10 +380,10 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint32_t t_o = tmem_base + (i == 0 ? Cfg::kColO0 : Cfg::kColO1) + hf * (D / 2) + lane_base;
     // At head dim 128 the loop's barriers go by 32-bit addresses that are worked out once; by pointers, which are converted where
     // they are used, 1 to 3 % slower (us, behind lasting load: 4 x 32 x 4096 977 : 960, causal 548 : 534, 1 x 32 x 16384 causal
-    // 1933 : 1904).  At head dim 64 it is the other way round (8 x 16 x 4096 715 : 728, 16 x 16 x 1024 107.6 : 110).
+    // 1933 : 1904; as a pair 977 : 941).  At head dim 64 it is the other way round (8 x 16 x 4096 715 : 728, 16 x 16 x 1024 107.6 : 110).
     auto bar_ref = [&](uint64_t* bar) {
       if constexpr (D == 64) return bar;
-      else return smem_u32(bar);
+      else return leader(bar);
     };
     const auto p_bar = bar_ref(p_full + i * Cfg::kPChunks);
     const uint32_t s_bar = smem_u32(s_full + i);
@@ -385,7 +414,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const DuoItem it = decode(idx);
         n_i = i ? it.n1 : it.n0;
         if (n_i == 0) continue;
-        const int row = it.m0 + i * Cfg::BM;
+        const int row = it.m0 + i * tile_rows + row_off;
         // the first steps see every key of their tile
         n_full = seq_k / BN;
         if (causal) n_full = (row + 1) / BN < n_full ? (row + 1) / BN : n_full;
@@ -451,7 +480,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           if (lane == 0) arrive_on(bar_ref(o_free + i));
         }
         const int col = hf * (D / 2) + c;  // first column of these 32
-        uint8_t* panel_row = stage_smem + (col >> 6) * Cfg::kQPanelBytes + r * 128;
+        uint8_t* panel_row = stage_smem + (Cfg::kStageTiles == 2 ? i * Cfg::kQTileBytes : 0) + (col >> 6) * Cfg::kQPanelBytes + r * 128;
 #pragma unroll
         for (int x = 0; x < 32; x += 8) {
           uint4 v4;
@@ -465,12 +494,12 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(stage_full);
+      if (lane == 0) mbar_arrive(stage_full + (Cfg::kStageTiles == 2 ? i : 0));
       if (lse != nullptr && hf == 0) {
         int again = idx;
         asm volatile("" : "+r"(again));  // worked out again here instead of kept through the steps
         const DuoItem it = decode(again);
-        const int row = it.m0 + i * Cfg::BM + r;
+        const int row = it.m0 + i * tile_rows + row_off + r;
         if (row < seq_len)
           lse[(static_cast<size_t>(it.b) * num_heads + it.h) * seq_len + row] =
               l_run > 0.f ? (m_ref * scale_log2 + log2f(l_run)) * 0.69314718055994531f : -INFINITY;
@@ -569,22 +598,28 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     set_max_regs_dec<Cfg::kRegsOther>();
     if (!SPLIT && warp == 18 && lane == 0) {
       // ============================================================= stores of finished tiles
-      uint32_t stores = 0;
+      uint32_t stores = 0;      // parity of the stores from each staging tile
       mbar_arrive(stage_free);  // the first store is a tile 0's (every item has one)
+      if (Cfg::kStageTiles == 2) mbar_arrive(stage_free + 1);
       for (int k = 0, idx = pos(0); idx < idx_end; idx = SPLIT ? idx_end : pos(++k)) {
         const DuoItem it = decode(idx);
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
           if ((i ? it.n1 : it.n0) == 0) continue;
-          mbar_wait(stage_full, stores & 1, abort_flag, 0x341 + i, idx);
+          const int tile = Cfg::kStageTiles == 2 ? i : 0;
+          mbar_wait(stage_full + tile, (stores >> tile) & 1, abort_flag, 0x341 + i, idx);
+          stores ^= 1u << tile;
           if (*abort_flag != 0) break;
+          const int row0 = it.m0 + i * tile_rows + row_off;
+          if (CTAS == 1 || row0 < seq_len) {  // of a pair's tile, the second CTA's rows may all be past the last query
 #pragma unroll
-          for (int p = 0; p < Cfg::kPanels; ++p)
-            tma_store_4d(&tm_o, stage_smem + p * Cfg::kQPanelBytes, p * 64, it.m0 + i * Cfg::BM, it.h, it.b);
-          tma_store_commit();
-          tma_store_wait_read();
-          mbar_arrive(stage_free + (i == 0 && it.n1 > 0));  // whose store comes next: this item's tile 1, or an item's tile 0
-          ++stores;
+            for (int p = 0; p < Cfg::kPanels; ++p)
+              tma_store_4d(&tm_o, stage_smem + tile * Cfg::kQTileBytes + p * Cfg::kQPanelBytes, p * 64, row0, it.h, it.b);
+            tma_store_commit();
+            tma_store_wait_read();
+          }
+          // whose store comes next: with one staging tile, this item's tile 1 or an item's tile 0
+          mbar_arrive(stage_free + (Cfg::kStageTiles == 2 ? i : (i == 0 && it.n1 > 0)));
         }
       }
     } else if (warp == 17 && lane == 0) {
@@ -595,41 +630,51 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const DuoItem it = decode(idx);
         const int h_kv = it.h / kv_group;
         const int n_max = it.n0 > it.n1 ? it.n0 : it.n1;
+        auto load = [&](void* dst, const CUtensorMap* tm, uint64_t* bar, int c0, int c1, int c2, int c3) __attribute__((always_inline)) {
+          if constexpr (CTAS == 2) tma_load_4d_pair(dst, tm, leader(bar), c0, c1, c2, c3);
+          else tma_load_4d(dst, tm, bar, c0, c1, c2, c3);
+        };
         auto load_q = [&](int i) __attribute__((always_inline)) {
           if ((i ? it.n1 : it.n0) > 0) {
             const uint32_t cnt = i ? q_cnt1 : q_cnt0;
             if (cnt > 0) mbar_wait(q_free + i, (cnt - 1) & 1, abort_flag, 0x402 + i, idx);
-            mbar_expect_tx(q_full + i, Cfg::kQTileBytes);
+            if (rank == 0) mbar_expect_tx(q_full + i, CTAS * Cfg::kQTileBytes);
 #pragma unroll
             for (int p = 0; p < Cfg::kPanels; ++p)
-              tma_load_4d(q_smem + i * Cfg::kQTileBytes + p * Cfg::kQPanelBytes, &tm_q, q_full + i, p * 64,
-                          it.m0 + i * Cfg::BM, it.h, it.b);
+              load(q_smem + i * Cfg::kQTileBytes + p * Cfg::kQPanelBytes, &tm_q, q_full + i, p * 64,
+                   it.m0 + i * tile_rows + row_off, it.h, it.b);
             if (i) ++q_cnt1; else ++q_cnt0;
           }
         };
         load_q(0);
         for (int t = 0; t < 2 * n_max; ++t) {
-          const int slot = t_run % STAGES;
-          const uint32_t ph = (t_run / STAGES) & 1;
+          const int slot = t_run % RING;
+          const uint32_t ph = (t_run / RING) & 1;
           mbar_wait(kv_empty + slot, ph ^ 1, abort_flag, 0x401, t);
           if (*abort_flag != 0) break;
-          mbar_expect_tx(kv_full + slot, Cfg::kKVTileBytes);
-          const CUtensorMap* tm = (t & 1) ? &tm_v : &tm_k;
+          if (rank == 0) mbar_expect_tx(kv_full + slot, Cfg::kKVTileBytes);
+          uint8_t* dst = kv_smem + slot * Cfg::kSlotBytes;
+          const int row = (it.j0 + (t >> 1)) * BN;
+          if (t & 1) {
 #pragma unroll
-          for (int p = 0; p < Cfg::kPanels; ++p)
-            tma_load_4d(kv_smem + slot * Cfg::kKVTileBytes + p * Cfg::kKVPanelBytes, tm, kv_full + slot, p * 64,
-                        (it.j0 + (t >> 1)) * BN, h_kv, it.b);
+            for (int p = 0; p < Cfg::kVPanels; ++p)
+              load(dst + p * Cfg::kKVPanelBytes, &tm_v, kv_full + slot, (rank * Cfg::kVPanels + p) * 64, row, h_kv, it.b);
+          } else {
+#pragma unroll
+            for (int p = 0; p < Cfg::kPanels; ++p)
+              load(dst + p * Cfg::kKPanelBytes, &tm_k, kv_full + slot, p * 64, row + rank * Cfg::kKRows, h_kv, it.b);
+          }
           ++t_run;
           if (t == 0) load_q(1);
         }
         if (*abort_flag != 0) break;
       }
-    } else if (warp == 16) {
+    } else if (warp == 16 && rank == 0) {
       // ============================================================= MMA issue (whole warp, one elected lane issues)
       constexpr uint64_t kDescK = smem_desc_sw128(16, 1024);
       constexpr uint64_t kDescV = smem_desc_sw128(Cfg::kKVPanelBytes, 1024);
-      constexpr uint32_t kIdescQK = idesc_f16_f32(Cfg::BM, BN, false, false);
-      constexpr uint32_t kIdescPV = idesc_f16_f32(Cfg::BM, D, false, true);
+      constexpr uint32_t kIdescQK = idesc_f16_f32(CTAS * Cfg::BM, BN, false, false);
+      constexpr uint32_t kIdescPV = idesc_f16_f32(CTAS * Cfg::BM, D, false, true);
       const uint32_t q_addr = smem_u32(q_smem);
       const uint32_t kv_addr = smem_u32(kv_smem);
       // One copy of the issue code per query tile (constant descriptors and columns) or one for both.  One elected lane issues
@@ -646,30 +691,30 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // read from lane 0, so that the compiler knows it to be the same in all lanes
       const uint32_t tmem_cols = __shfl_sync(0xffffffffu, tmem_base, 0);
       auto wait_kv = [&](uint32_t t_abs, int j) __attribute__((always_inline)) {
-        mbar_wait(kv_full + t_abs % STAGES, (t_abs / STAGES) & 1, abort_flag, 0x501, j);
+        mbar_wait(kv_full + t_abs % RING, (t_abs / RING) & 1, abort_flag, 0x501, j);
       };
       // S_i(j) = Q_i . K_j^T of item `it` (ring index t_abs)
       auto issue_qk = [&](int i, const DuoItem& it, int j, uint32_t t_abs) __attribute__((always_inline)) {
-        const int slot = t_abs % STAGES;
+        const int slot = t_abs % RING;
         tc_fence_after_sync();
         const uint64_t q_d = smem_desc_at(kDescK, q_addr + i * Cfg::kQTileBytes);
-        const uint64_t k_d = smem_desc_at(kDescK, kv_addr + slot * Cfg::kKVTileBytes);
+        const uint64_t k_d = smem_desc_at(kDescK, kv_addr + slot * Cfg::kSlotBytes);
         const uint32_t t_s = tmem_cols + (i == 0 ? Cfg::kColS0 : Cfg::kColS1);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t qoff = ((kk >> 2) * Cfg::kQPanelBytes + (kk & 3) * 32) >> 4;
-            const uint32_t koff = ((kk >> 2) * Cfg::kKVPanelBytes + (kk & 3) * 32) >> 4;
-            mma_ss(t_s, q_d + qoff, k_d + koff, kIdescQK, kk > 0);
+            const uint32_t koff = ((kk >> 2) * Cfg::kKPanelBytes + (kk & 3) * 32) >> 4;
+            mma_ss_g<CTAS>(t_s, q_d + qoff, k_d + koff, kIdescQK, kk > 0);
           }
-          mma_commit(s_full + i);
-          if ((i == 1) || !(j < it.n1)) mma_commit(kv_empty + slot);
-          if (j + 1 == (i ? it.n1 : it.n0)) mma_commit(q_free + i);
+          mma_commit_g<CTAS>(s_full + i);
+          if ((i == 1) || !(j < it.n1)) mma_commit_g<CTAS>(kv_empty + slot);
+          if (j + 1 == (i ? it.n1 : it.n0)) mma_commit_g<CTAS>(q_free + i);
         }
         __syncwarp();
       };
       auto issue_pv = [&](int i, const DuoItem& it, int j, uint32_t t_abs) __attribute__((always_inline)) {
-        const int slot = t_abs % STAGES;
+        const int slot = t_abs % RING;
         const bool last = j + 1 == (i ? it.n1 : it.n0);
         wait_kv(t_abs, j);
         if (j == 0) {
@@ -678,7 +723,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           phases ^= 0x10u << i;
         }
         if (!last) wait_kv(t_abs + 1, j);  // the next K tile: ahead of P, off the path to the next scores
-        const uint64_t v_d = smem_desc_at(kDescV, kv_addr + slot * Cfg::kKVTileBytes);
+        const uint64_t v_d = smem_desc_at(kDescV, kv_addr + slot * Cfg::kSlotBytes);
         const uint32_t t_p = tmem_cols + (i == 0 ? Cfg::kColS0 : Cfg::kColS1);
         const uint32_t t_o = tmem_cols + (i == 0 ? Cfg::kColO0 : Cfg::kColO1);
         const uint32_t ph = (phases >> i) & 1;
@@ -691,11 +736,11 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             for (int s2 = 0; s2 < 4; ++s2) {
               // 16 keys per MMA: the chunk's 32 keys of either half; a half's P sits in columns [0,32) / [64,96)
               const int kk = (s2 >> 1) * 4 + q * 2 + (s2 & 1);
-              mma_ts(t_o, t_p + (kk >> 2) * 64 + (kk & 3) * 8, v_d + ((kk * 2048) >> 4), kIdescPV, (j > 0 || q > 0 || s2 > 0));
+              mma_ts_g<CTAS>(t_o, t_p + (kk >> 2) * 64 + (kk & 3) * 8, v_d + ((kk * 2048) >> 4), kIdescPV, (j > 0 || q > 0 || s2 > 0));
             }
             if (q == Cfg::kPChunks - 1) {
-              if (last) mma_commit(o_full + i);
-              if ((i == 1) || !(j < it.n1)) mma_commit(kv_empty + slot);
+              if (last) mma_commit_g<CTAS>(o_full + i);
+              if ((i == 1) || !(j < it.n1)) mma_commit_g<CTAS>(kv_empty + slot);
             }
           }
           __syncwarp();
@@ -763,6 +808,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (*abort_flag == 1u) settle_after_abort();
   tc_fence_before_sync();
   __syncthreads();
+  if constexpr (CTAS == 2) cluster_sync_all();  // neither CTA leaves while the other may still signal it
   if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
   if constexpr (SPLIT) {
     __syncwarp();
@@ -789,13 +835,12 @@ inline bool duo_heaviest_first(bool causal, const AttnShape& shp, const AttnShap
 // same number of steps per round of two items, and what is left is the incomplete last round: taken where that is 5 % at most.
 // The slices under way at a time are twice as many as slice by slice, but still few.
 // us, behind lasting load, slice by slice -> matched: 4 x 32 x 4096 x 128 578 -> 558, 1 x 32 x 16384 2043 -> 1967.
-inline bool duo_matched(bool causal, const AttnShape& shp, const AttnShape& shp_kv, int n_pairs, int sms, int max_deal) {
-  const long long slices = static_cast<long long>(shp.B) * shp.H, items = slices * n_pairs;
+inline bool duo_matched(bool causal, const AttnShape& shp, const AttnShape& shp_kv, long long items, int units, int max_deal) {
   if (!causal || shp.S <= 1024 || shp.S > ((shp_kv.S + 127) / 128) * 128 || (items & 1) != 0 || items >= (1LL << 30) ||
       duo_heaviest_first(causal, shp, shp_kv))
     return false;
-  const long long twos = items / 2, rounds = (twos + sms - 1) / sms;
-  return twos >= sms && 2 * rounds < max_deal && 100 * rounds * sms <= 105 * twos;
+  const long long twos = items / 2, rounds = (twos + units - 1) / units;
+  return twos >= units && 2 * rounds < max_deal && 100 * rounds * units <= 105 * twos;
 }
 
 // CTAs per work item for a problem of few items: the cluster size whose rounds take the fewest KV steps, counting 3 steps for a
@@ -822,25 +867,49 @@ inline int duo_parts(int items, int steps, bool causal, int sms, const int (&act
 // what duo_parts needs from the device costs it 0.1 to 0.2 us a call (4 heads of 256 rows: 6.20 -> 6.00 us).
 inline bool duo_may_split(int items, int steps, int sms) { return 2 * items <= sms && steps > 4; }
 
+// Whether CTA pairs take the items, by rows (items of 512) or by heads (items of 256 rows of two heads of a K/V head's group).
+//
+// A pair's products read half as much of K and V from shared memory, and half as much of them is copied into it: products and copies
+// alone take 2106 cycles per 128 keys of two tiles instead of 2586 (of 2048 at the tensor pipe's rate: shared memory is full in
+// single CTAs, whose scores' operands alone ask for its 128 bytes a cycle).  The chain through the softmax, 2900 cycles, does not get
+// shorter by it, but the board, which is at its power limit in long calls, runs 3 % faster.  So it pays in long calls; in short ones
+// the pair's start, end and common pace cost more (behind 15 ms of load instead of 60, up to 120 us: 1.00 to 1.07 times as long).
+// us, single CTAs -> pairs, behind lasting load: 4 x 32 x 4096 993 -> 973, 16 x 16 x 1024 148 -> 147, 2 x 32 x 2325 203 -> 198,
+// causal, by heads: 2 x 32/8 x 3000 164 -> 161, 4 x 40/20 x 2895 411 -> 389, 9 x 40/20 x 1741 358 -> 345; of 71 drawn calls that
+// the rule takes 0.946 to 0.992 times as long.  What it leaves:
+//   * items of 512 rows that need more rounds (1 x 40 x 2610: 1.14, 5 x 40 x 1130: 1.08; by heads they never do);
+//   * fewer than 48 steps of two tiles per SM, or items of fewer than 8 steps (16 x 40 x 3490 on 116 keys: 1.06);
+//   * causal items by rows, whose second pair of tiles works alone for two steps instead of one (4 x 32 x 4096 534 -> 552).
+enum DuoPair : int { kDuoSingle = 0, kDuoPairRows = 1, kDuoPairHeads = 2 };
+inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int steps, int sms) {
+  const bool heads = group % 2 == 0;
+  if ((causal && !heads) || steps < 8) return kDuoSingle;
+  const long long items = static_cast<long long>(slices) * ((seq_len + 255) / 256);
+  const long long pair_items = heads ? items / 2 : static_cast<long long>(slices) * ((seq_len + 511) / 512);
+  const int pairs = sms / 2;
+  if (pairs <= 0 || (pair_items + pairs - 1) / pairs > (items + sms - 1) / sms) return kDuoSingle;
+  if (items * (causal ? (steps + 1) / 2 : steps) < 48LL * sms) return kDuoSingle;
+  return heads ? kDuoPairHeads : kDuoPairRows;
+}
+
 // How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit).
 struct DuoPlan {
   DuoMode mode;
+  DuoPair pair;
   int parts, sms, items, n_pairs, n_kv;
 };
 
 template <int D, int STAGES>
 inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, cudaStream_t stream, DuoPlan& plan) {
   using Cfg = DuoCfg<D, STAGES>;
-  plan.mode = kDuoDealt;
-  plan.parts = 1;
-  plan.sms = device_sm_count();
+  plan = DuoPlan{kDuoDealt, kDuoSingle, 1, device_sm_count(), 0, 0, 0};
   if (plan.sms <= 0) return kAttnLaunchFailed;
   plan.n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
   plan.n_kv = (shp_kv.S + Cfg::BN - 1) / Cfg::BN;
   plan.items = plan.n_pairs * shp.B * shp.H;
   const int steps = causal && 2 * plan.n_pairs < plan.n_kv ? 2 * plan.n_pairs : plan.n_kv;
   if (duo_may_split(plan.items, steps, plan.sms)) {
-    auto split = attn_fwd_duo_kernel<D, STAGES, kDuoSplit>;
+    auto split = attn_fwd_duo_kernel<D, STAGES, kDuoSplit, 1>;
     struct Tag {};
     const int rc = ensure_dynamic_smem<Tag>(split, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
     if (rc != kAttnOk) return rc;
@@ -849,10 +918,41 @@ inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, 
     if (active == nullptr) return kAttnLaunchFailed;
     plan.parts = duo_parts(plan.items, steps, causal, plan.sms, *active);
     if (plan.parts > 1) plan.mode = kDuoSplit;
-  } else if (duo_matched(causal, shp, shp_kv, plan.n_pairs, plan.sms, Cfg::kMaxDeal)) {  // two items per SM and more
-    plan.mode = kDuoMatched;
+  } else {
+    int units = plan.sms, max_deal = Cfg::kMaxDeal;
+    if constexpr (D == 128) {
+      plan.pair = duo_pair(causal, shp.B * shp.H, shp.H / shp_kv.H, shp.S, steps, plan.sms);
+      if (plan.pair != kDuoSingle) {
+        if (plan.pair == kDuoPairRows) plan.n_pairs = (shp.S + 4 * Cfg::BM - 1) / (4 * Cfg::BM);
+        plan.items = plan.n_pairs * shp.B * shp.H / (plan.pair == kDuoPairHeads ? 2 : 1);
+        units = plan.sms / 2;
+        max_deal = DuoCfg<D, STAGES, 2>::kMaxDeal;
+      }
+    }
+    if (duo_matched(causal, shp, shp_kv, plan.items, units, max_deal)) plan.mode = kDuoMatched;  // two items per SM and more
   }
   return kAttnOk;
+}
+
+template <int D, int STAGES, DuoMode MODE, int CTAS>
+inline int launch_duo_dealt(const DuoPlan& plan, cudaStream_t stream, const CUtensorMap& tm_q, const CUtensorMap& tm_k,
+                            const CUtensorMap& tm_v, const CUtensorMap& tm_o, const AttnShape& shp, const AttnExtras& ex, bool causal,
+                            float scale_log2, bool heaviest_first) {
+  using Cfg = DuoCfg<D, STAGES, CTAS>;
+  auto kernel = attn_fwd_duo_kernel<D, STAGES, MODE, CTAS>;
+  struct Tag {};
+  const int rc = ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
+  if (rc != kAttnOk) return rc;
+  const int units = plan.sms / CTAS;
+  const int clusters = plan.items < units ? plan.items : units;
+  auto launch = [&](auto... args) {
+    if constexpr (CTAS == 1) return launch_overlapped(kernel, dim3(clusters), Cfg::kThreads, Cfg::kSmemBytes, stream, args...);
+    ClusterLaunch cluster(clusters, Cfg::kThreads, Cfg::kSmemBytes, stream);
+    cluster.set_ctas(CTAS);
+    return cluster(kernel, args...);
+  };
+  return launch(tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0, scale_log2, ex.kv_group, ex.lse, ex.seq_k,
+                heaviest_first ? 1 : 0, plan.n_kv, plan.n_pairs, plan.items, 1, plan.pair == kDuoPairHeads ? 1 : 0, DuoOut{});
 }
 
 // Host launcher for the kernel with two softmax threads per row. Returns an AttnReturnCode.
@@ -865,36 +965,35 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
   CUtensorMap tm_q, tm_k, tm_v, tm_o;
   int rc = cached_attn_tensor_map(&tm_q, q, shp, st[0], Cfg::BM);
   if (rc != kAttnOk) return rc;
-  rc = cached_attn_tensor_map(&tm_k, k, shp_kv, st[1], Cfg::BN);
+  DuoPlan plan;
+  rc = duo_plan<D, STAGES>(shp, shp_kv, causal, stream, plan);
+  if (rc != kAttnOk) return rc;
+  rc = cached_attn_tensor_map(&tm_k, k, shp_kv, st[1], plan.pair == kDuoSingle ? Cfg::BN : Cfg::BN / 2);
   if (rc != kAttnOk) return rc;
   rc = cached_attn_tensor_map(&tm_v, v, shp_kv, st[2], Cfg::BN);
   if (rc != kAttnOk) return rc;
   rc = cached_attn_tensor_map(&tm_o, o, shp, st[3], Cfg::BM);
   if (rc != kAttnOk) return rc;
 
-  DuoPlan plan;
-  rc = duo_plan<D, STAGES>(shp, shp_kv, causal, stream, plan);
-  if (rc != kAttnOk) return rc;
   const float scale_log2 = scale * 1.44269504088896340736f;
   if (plan.mode == kDuoSplit) {
     ClusterLaunch launch(plan.items, Cfg::kThreads, Cfg::kSmemBytes, stream);
     launch.set_ctas(plan.parts);
     const DuoOut out{o, shp.B > 1 ? st[3].b : 0, shp.H > 1 ? st[3].h : 0, shp.S > 1 ? st[3].s : 0};
-    return launch(attn_fwd_duo_kernel<D, STAGES, kDuoSplit>, tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0,
-                  scale_log2, ex.kv_group, ex.lse, ex.seq_k, 1, plan.n_kv, plan.n_pairs, plan.items, plan.parts, out);
+    return launch(attn_fwd_duo_kernel<D, STAGES, kDuoSplit, 1>, tm_q, tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0,
+                  scale_log2, ex.kv_group, ex.lse, ex.seq_k, 1, plan.n_kv, plan.n_pairs, plan.items, plan.parts, 0, out);
   }
-  auto kernel = attn_fwd_duo_kernel<D, STAGES, kDuoDealt>;
-  if (plan.mode == kDuoMatched) {
-    struct Tag {};
-    kernel = attn_fwd_duo_kernel<D, STAGES, kDuoMatched>;
-    rc = ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
-  } else {
-    rc = ensure_dynamic_smem<Cfg>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
-  }
-  if (rc != kAttnOk) return rc;
-  return launch_overlapped(kernel, dim3(plan.items < plan.sms ? plan.items : plan.sms), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q,
-                           tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0, scale_log2, ex.kv_group, ex.lse, ex.seq_k,
-                           duo_heaviest_first(causal, shp, shp_kv) ? 1 : 0, plan.n_kv, plan.n_pairs, plan.items, 1, DuoOut{});
+  const bool heaviest_first = duo_heaviest_first(causal, shp, shp_kv);
+  auto dealt = [&](auto mode, auto ctas) {
+    return launch_duo_dealt<D, STAGES, decltype(mode)::value, decltype(ctas)::value>(plan, stream, tm_q, tm_k, tm_v, tm_o, shp, ex, causal,
+                                                                                      scale_log2, heaviest_first);
+  };
+  using Dealt = std::integral_constant<DuoMode, kDuoDealt>;
+  using Matched = std::integral_constant<DuoMode, kDuoMatched>;
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, D == 128 ? 2 : 1>;  // head dim 64 has no pairs
+  if (plan.pair != kDuoSingle) return plan.mode == kDuoMatched ? dealt(Matched{}, Two{}) : dealt(Dealt{}, Two{});
+  return plan.mode == kDuoMatched ? dealt(Matched{}, One{}) : dealt(Dealt{}, One{});
 }
 
 }  // namespace sm100

@@ -1,0 +1,46 @@
+"""Which calls the row-pair kernel's launcher gives to CTA pairs: the rule, which is host code, at its edges."""
+import importlib
+
+import pytest
+
+op = importlib.import_module("fray_b200.jit_kernels.flashattn_cute")
+SINGLE, ROWS, HEADS = 0, 1, 2
+
+
+@pytest.fixture(scope="module")
+def pair(tmp_path_factory):
+    from fray_b200.jit import build, generate
+    args = (("n", int),)
+    code = generate(op.includes, args, "\n__return_code = 0;\n", """
+extern "C" EXPORT_API int pair(int causal, int slices, int group, int seq_len, int steps, int sms) {
+    return fray::sm100::duo_pair(causal != 0, slices, group, seq_len, steps, sms);
+}
+""")
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setenv("FRAY_CACHE_DIR", str(tmp_path_factory.mktemp("pair")))
+        return build("pair_rule", args, code).symbol("pair")
+
+
+def test_calls_the_rule_takes(pair):
+    assert pair(0, 128, 1, 4096, 32, 148) == ROWS and pair(0, 256, 1, 1024, 8, 148) == ROWS   # 0.98, 0.99
+    assert pair(1, 64, 4, 3000, 24, 148) == HEADS and pair(1, 160, 2, 2895, 23, 148) == HEADS  # 0.98, 0.95
+    assert pair(0, 148, 2, 600, 17, 148) == HEADS  # heads that could not be laid end to end
+
+
+def test_calls_the_rule_leaves(pair):
+    assert pair(1, 128, 1, 4096, 32, 148) == SINGLE and pair(1, 128, 3, 4096, 32, 148) == SINGLE  # causal items by rows: 1.03
+    assert pair(0, 40, 1, 2610, 39, 148) == SINGLE   # 240 items of 512 rows on 74 pairs take a fourth round: 1.14
+    assert pair(0, 640, 1, 3490, 1, 148) == SINGLE   # 1.06
+    assert pair(0, 32, 1, 2048, 16, 148) == SINGLE   # 28 steps per SM: level, and 1.01 on a cooler board
+
+
+def test_pairs_never_need_more_rounds(pair):
+    for slices in range(2, 400, 2):
+        for seq_len in (200, 256, 257, 512, 513, 700, 1024, 1100):
+            for group in (1, 2):
+                form = pair(0, slices, group, seq_len, 64, 148)
+                items = slices * -(-seq_len // 256)
+                if form != SINGLE:
+                    mine = items // 2 if form == HEADS else slices * -(-seq_len // 512)
+                    assert -(-mine // 74) <= -(-items // 148) and (form == HEADS) == (group == 2)
+    assert pair(0, 400, 2, 4096, 64, 1) == SINGLE  # a device without a pair of SMs
