@@ -89,7 +89,8 @@ struct DuoCfg {
   // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
   static constexpr int kMaxDeal = CTAS == 2 ? 140 : 190;
   static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
-  static constexpr int kSmemBytes = kUsedBytes;
+  // slack for the split form, which brings the dynamic segment to a 1024-byte boundary itself (its base is one already; checked)
+  static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
   static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
   static constexpr int kPartStride = D + 4;  // SPLIT: floats from row to row of the partial results
   static constexpr int kOffPartMl = 2 * BM * kPartStride * 4;
@@ -230,8 +231,19 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   constexpr int RING = Cfg::kRing;
   constexpr bool SPLIT = MODE == kDuoSplit;
   static_assert(CTAS == 1 || !SPLIT, "a split item's clusters are of single CTAs");
-  extern __shared__ __align__(1024) uint8_t duo_smem[];  // aligned by declaration: every address in it is a constant
-  uint8_t* smem = duo_smem;
+  uint8_t* smem;
+  bool fits;
+  if constexpr (SPLIT) {  // rounded up here, and the loop's barriers by pointers: 2 slices of 264 rows on 1913 keys 15.2 us, 15.5 as below
+    extern __shared__ uint8_t duo_raw[];
+    const uint32_t raw_addr = smem_u32(duo_raw);
+    const uint32_t align_off = ((raw_addr + 1023u) & ~1023u) - raw_addr;
+    smem = duo_raw + align_off;
+    fits = align_off + Cfg::kUsedBytes <= Cfg::kSmemBytes;
+  } else {
+    extern __shared__ __align__(1024) uint8_t duo_smem[];  // aligned by declaration: every address in it is a constant
+    smem = duo_smem;
+    fits = (smem_u32(smem) & 1023u) == 0;
+  }
   uint8_t* q_smem = smem + Cfg::kOffQ;
   uint8_t* kv_smem = smem + Cfg::kOffKV;
   uint8_t* stage_smem = smem + Cfg::kOffStage;
@@ -259,7 +271,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  if ((smem_u32(smem) & 1023u) != 0) {  // never seen
+  if (!fits) {  // never seen: the segment's base is 1024-byte aligned
     if (tid == 0) atomicCAS(&fray_attn_status[0], 0, 0x601);
     return;
   }
@@ -382,7 +394,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // they are used, 1 to 3 % slower (us, behind lasting load: 4 x 32 x 4096 977 : 960, causal 548 : 534, 1 x 32 x 16384 causal
     // 1933 : 1904; as a pair 977 : 941).  At head dim 64 it is the other way round (8 x 16 x 4096 715 : 728, 16 x 16 x 1024 107.6 : 110).
     auto bar_ref = [&](uint64_t* bar) {
-      if constexpr (D == 64) return bar;
+      if constexpr (D == 64 || SPLIT) return bar;
       else return leader(bar);
     };
     const auto p_bar = bar_ref(p_full + i * Cfg::kPChunks);
@@ -405,7 +417,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // phase parities, toggled: bit 0 s_full, bit 1 o_full, bit 2 stage_free
     uint32_t phases = 0;
     auto wait_scores = [&](int j) __attribute__((always_inline)) {
-      if constexpr (D == 64) mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
+      if constexpr (D == 64 || SPLIT) mbar_wait(s_full + i, phases & 1, abort_flag, 0x201 + i, j);
       else mbar_wait(s_bar, phases & 1, abort_flag, 0x201 + i, j);
     };
     for (int k = 0, idx = pos(0); idx < idx_end; idx = SPLIT ? idx_end : pos(++k)) {
