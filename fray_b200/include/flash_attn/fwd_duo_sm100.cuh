@@ -9,6 +9,7 @@
 //   warp 17     TMA producer (Q tiles, K_j, V_j through a ring of STAGES buffers)
 //   warp 18     TMA stores of finished tiles
 //   warp 19     idle (fills the warpgroup for setmaxnreg)
+// At head dim 64 most calls go to four independent streams per CTA instead (duo_quad, four_streams_sm100.cuh).
 // At head dim 128 long calls put a pair of CTAs to an item (duo_pair): two query tiles in each of the two, every product one
 // cta_group::2 instruction that the leader's warp 16 issues for both, each CTA with half of K's rows and of V's columns.
 //
@@ -46,6 +47,7 @@
 
 #include <type_traits>
 
+#include "four_streams_sm100.cuh"
 #include "host_sm100.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_tile_sm100.cuh"
@@ -102,10 +104,6 @@ struct DuoCfg {
   static constexpr int kRegsTotal = 512 * kRegsSoftmax + 128 * kRegsOther;
   static_assert(kRegsTotal <= kThreads * kRegsLaunch, "register budgets exceed the CTA's allocation");
 };
-
-// Arrives on a barrier: of this CTA, or by its cluster-wide address.
-__device__ __forceinline__ void arrive_on(uint64_t* bar) { mbar_arrive(bar); }
-__device__ __forceinline__ void arrive_on(uint32_t cluster_addr) { mbar_arrive_cluster(cluster_addr); }
 
 // Meets the barrier and returns whether any of its threads passed `p`.
 __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
@@ -904,6 +902,16 @@ inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int ste
   return heads ? kDuoPairHeads : kDuoPairRows;
 }
 
+// Head dim 64: whether the items go to the kernel with four independent streams per CTA (four_streams_sm100.cuh) instead.  Of
+// 105 drawn calls that the rule sends there (1 to 46 steps, 80 to 4800 items, with and without a causal mask) it took 0.84 to 1.01
+// times as long, 0.92 on average.  What it loses are many short items that all end with whole steps, where its
+// end of an item, which adds up two accumulators, weighs more than its finer steps gain: 16 x 16 x 1024 with large logits 113 : 110
+// us, 32 x 16 x 512 62.9 : 61.9, 256 keys 39.1 : 38.3, 511 rows on 194 keys 23.7 : 22.7; 1280 keys 122.1 : 122.6.
+inline bool duo_quad(bool causal, long long items, int seq_k, int sms) {
+  const bool whole_steps = (seq_k + 63) / 64 % 2 == 0;  // the last 128 keys are more than half there
+  return causal || !whole_steps || seq_k > 1024 || 2 * items < 5LL * sms;
+}
+
 // How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit).
 struct DuoPlan {
   DuoMode mode;
@@ -996,16 +1004,23 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
                   scale_log2, ex.kv_group, ex.lse, ex.seq_k, 1, plan.n_kv, plan.n_pairs, plan.items, plan.parts, 0, out);
   }
   const bool heaviest_first = duo_heaviest_first(causal, shp, shp_kv);
-  auto dealt = [&](auto mode, auto ctas) {
-    return launch_duo_dealt<D, STAGES, decltype(mode)::value, decltype(ctas)::value>(plan, stream, tm_q, tm_k, tm_v, tm_o, shp, ex, causal,
-                                                                                      scale_log2, heaviest_first);
-  };
-  using Dealt = std::integral_constant<DuoMode, kDuoDealt>;
-  using Matched = std::integral_constant<DuoMode, kDuoMatched>;
-  using One = std::integral_constant<int, 1>;
-  using Two = std::integral_constant<int, D == 128 ? 2 : 1>;  // head dim 64 has no pairs
-  if (plan.pair != kDuoSingle) return plan.mode == kDuoMatched ? dealt(Matched{}, Two{}) : dealt(Dealt{}, Two{});
-  return plan.mode == kDuoMatched ? dealt(Matched{}, One{}) : dealt(Dealt{}, One{});
+  if constexpr (D == 64) {
+    if (duo_quad(causal, plan.items, shp_kv.S, plan.sms))
+      return launch_attn_fwd_quad<D>(tm_q, tm_k, tm_v, tm_o, shp, ex, causal, scale_log2, heaviest_first, plan.mode == kDuoMatched,
+                                     plan.n_pairs, plan.items, plan.sms, stream);
+    return launch_duo_dealt<D, STAGES, kDuoDealt, 1>(plan, stream, tm_q, tm_k, tm_v, tm_o, shp, ex, causal, scale_log2, heaviest_first);
+  } else {
+    auto dealt = [&](auto mode, auto ctas) {
+      return launch_duo_dealt<D, STAGES, decltype(mode)::value, decltype(ctas)::value>(plan, stream, tm_q, tm_k, tm_v, tm_o, shp, ex, causal,
+                                                                                        scale_log2, heaviest_first);
+    };
+    using Dealt = std::integral_constant<DuoMode, kDuoDealt>;
+    using Matched = std::integral_constant<DuoMode, kDuoMatched>;
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    if (plan.pair != kDuoSingle) return plan.mode == kDuoMatched ? dealt(Matched{}, Two{}) : dealt(Dealt{}, Two{});
+    return plan.mode == kDuoMatched ? dealt(Matched{}, One{}) : dealt(Dealt{}, One{});
+  }
 }
 
 }  // namespace sm100
