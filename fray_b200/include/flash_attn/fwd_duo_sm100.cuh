@@ -91,7 +91,7 @@ struct DuoCfg {
   // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
   static constexpr int kMaxDeal = CTAS == 2 ? 140 : 190;
   static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
-  // slack for the split form, which brings the dynamic segment to a 1024-byte boundary itself (its base is one already; checked)
+  // slack for the forms that bring the dynamic segment to a 1024-byte boundary themselves (its base is one already; checked)
   static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
   static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
   static constexpr int kPartStride = D + 4;  // SPLIT: floats from row to row of the partial results
@@ -231,14 +231,17 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   static_assert(CTAS == 1 || !SPLIT, "a split item's clusters are of single CTAs");
   uint8_t* smem;
   bool fits;
-  if constexpr (SPLIT) {  // rounded up here, and the loop's barriers by pointers: 2 slices of 264 rows on 1913 keys 15.2 us, 15.5 as below
+  // Aligned by declaration every address in it is a constant, which the long items of the matched form and of pairs gain 1 % by
+  // (1 x 32 x 16384 causal 1930 -> 1912 us); short items lose (3 x 32 x 826 on 184 keys 21.8 : 23.6, 6 x 16 x 333 causal 16.8 :
+  // 17.5, split: 2 slices of 264 rows on 1913 keys 15.2 : 15.5), so the other forms round it up here.
+  if constexpr (SPLIT || (D == 128 && MODE == kDuoDealt && CTAS == 1)) {
     extern __shared__ uint8_t duo_raw[];
     const uint32_t raw_addr = smem_u32(duo_raw);
     const uint32_t align_off = ((raw_addr + 1023u) & ~1023u) - raw_addr;
     smem = duo_raw + align_off;
     fits = align_off + Cfg::kUsedBytes <= Cfg::kSmemBytes;
   } else {
-    extern __shared__ __align__(1024) uint8_t duo_smem[];  // aligned by declaration: every address in it is a constant
+    extern __shared__ __align__(1024) uint8_t duo_smem[];
     smem = duo_smem;
     fits = (smem_u32(smem) & 1023u) == 0;
   }
