@@ -36,11 +36,13 @@
 // 79, 16 x 16 x 1024 x 64 103 : 122, 16 x 16 x 1024 x 128 causal 105 : 127, 8 x 16 x 4096 x 64 721-726 : 801-807, 4 x 16 x 2048
 // x 64 causal 59 : 83; 20 launches of the first from an idle board 853-890 : 909-956 (with products issued as they are now:
 // 823-840, see the MMA warp).  2870 cycles per 128 keys of two tiles inside an item; an item costs 2 to 3 us beside its steps.
-// Tried and left out while products were still issued instruction by instruction, which kept the MMA warp busy for a tile's whole
-// step (so these show what lost then, not that it loses now): 12 or 25 % of the exponentials as a degree-5 polynomial on the FMA
-// pipe (-8 %), polling instead of suspending waits in the MMA warp or the softmax warps (level), 6 or 8 ring slots at head dim 64
-// (level), at head dim 64 a P buffer of its own, which breaks the chain but adds two barriers per step (716 : 690 us at
-// 8 x 16 x 4096), the second fetch of scores issued ahead of the first exponentials (-2 %).
+// Tried and left out (us or thousand cycles a CTA, 4 x 32 x 4096 behind lasting load unless noted): 6 to 25 % of the exponentials as
+// a polynomial of degree 4 or 5 on the FMA pipe (cycles level to -2 %, but the board is at its power limit: +2 to +5 %), the first 32
+// exponentials on trust, ahead of the halves' agreement (1326 -> 1366: those of the two tiles meet at the unit then), the MMA warp's
+// waits for K and V once per step (level), an issuing warp per query tile (975 -> 1111: the tiles' products interleave in the pipe), the
+// issuing role in one lane altogether (its operands are not known to be uniform then, 2 to 3 times as long), polling instead of
+// suspending waits (level), the second fetch of scores ahead of the first exponentials (-2 %).  The softmax alone takes 2746 cycles of
+// the step's 2960 with the items' ends and the products with their copies 2586, so what helps one of them alone does not show.
 //
 // Every barrier wait is bounded (see sm100_ptx.cuh), and what a warp does next never depends on whether a wait ran out, so
 // the named barriers always meet: a protocol error ends as a status word and a wrong answer, never as a hung GPU.
