@@ -847,15 +847,20 @@ inline bool duo_heaviest_first(bool causal, const AttnShape& shp, const AttnShap
 }
 
 // Slice by slice the busiest CTA of a causal problem has 6 to 25 % more steps than its share.  Matched by twos every CTA has the
-// same number of steps per round of two items, and what is left is the incomplete last round: taken where that is 5 % at most.
-// The slices under way at a time are twice as many as slice by slice, but still few.
-// us, behind lasting load, slice by slice -> matched: 4 x 32 x 4096 x 128 578 -> 558, 1 x 32 x 16384 2043 -> 1967.
+// same number of steps per round of two items, and what is left is the incomplete last round: taken where that is 13 % at
+// most, for grouped heads 5 %.  The slices under way at a time are twice as many as slice by slice, but still few.
+// us, behind lasting load, slice by slice -> matched: 4 x 32 x 4096 x 128 578 -> 558, 1 x 32 x 16384 2043 -> 1967.  58 shapes
+// of 5 to 13 % (1420 to 11577 rows, K and V of 130 to 465 MB, both head dims) took 0.68 to 1.01 of the time, half of them less
+// than 0.96: 2 x 16 x 10841 x 128 1200 -> 811, 8 x 32 x 3311 x 64 542 -> 533, 7 x 16 x 4653 x 64 472 -> 478; at 15 to 19 % 0.77
+// to 1.04 (8 x 12 x 3935 x 128 420 -> 439), and two query heads per K/V head from 5 % on 0.91 to 1.08 (5 x 32 x 6605 x 128
+// 1608 -> 1732).
 inline bool duo_matched(bool causal, const AttnShape& shp, const AttnShape& shp_kv, long long items, int units, int max_deal) {
   if (!causal || shp.S <= 1024 || shp.S > ((shp_kv.S + 127) / 128) * 128 || (items & 1) != 0 || items >= (1LL << 30) ||
       duo_heaviest_first(causal, shp, shp_kv))
     return false;
   const long long twos = items / 2, rounds = (twos + units - 1) / units;
-  return twos >= units && 2 * rounds < max_deal && 100 * rounds * units <= 105 * twos;
+  return twos >= units && 2 * rounds < max_deal &&
+         100 * rounds * units <= (shp.H == shp_kv.H ? 113 : 105) * twos;
 }
 
 // CTAs per work item for a problem of few items: the cluster size whose rounds take the fewest KV steps, counting 3 steps for a
