@@ -31,8 +31,9 @@
 // scores fetched again instead of kept (spills elsewhere, 3 % slower), the merge by the group that ends last while the other goes on
 // (400 bytes of spills, 10 % slower), tile 1 started behind tile 0 (level), offsets moved from 2^12 on instead of 2^8 (level).
 //
-// Every barrier wait is bounded (see sm100_ptx.cuh), and what a warp does next never depends on whether a wait ran out, so
-// the named barriers always meet.
+// Every barrier wait is bounded (see sm100_ptx.cuh).  A softmax warp goes through its items whether or not a wait ran out, so the
+// named barriers always meet; producer, stores and issue stop at a step, a tile or an item of their own, the issuing warps as whole
+// warps.
 
 #include <type_traits>
 
@@ -524,7 +525,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           if (s_i == 0)
             for (int g = 0; g < 2; ++g) first_scores(g);
           if (row < 0) break;
-          if (*abort_flag != 0) break;
+          if (__any_sync(0xffffffffu, *abort_flag != 0)) break;  // by vote: item_row and the elections need every lane
           n = nn;
           s_max = s_nxt;
           t_base = t_next;
