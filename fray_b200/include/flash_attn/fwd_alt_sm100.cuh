@@ -327,8 +327,8 @@ attn_fwd_alt_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (stop != 0) return;  // an earlier launch left the device status raised
 
   if (warp == 0) {
-    tmem_alloc(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish();
+    tmem_alloc(tmem_slot, Cfg::kTmemCols, CtaGroup<CTAS>{});
+    tmem_relinquish(CtaGroup<CTAS>{});
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -656,7 +656,7 @@ attn_fwd_alt_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync_all();  // neither CTA leaves while the other may still signal it
-  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols, CtaGroup<CTAS>{});
 #ifdef FRAY_ATTN_TRACE
   if (tid == 0) FRAY_TRACE(6, 0, 2);
   __syncthreads();

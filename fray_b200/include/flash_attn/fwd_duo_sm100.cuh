@@ -350,8 +350,8 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   __syncwarp();
   if (warp == 0) {
-    tmem_alloc(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish();
+    tmem_alloc(tmem_slot, Cfg::kTmemCols, CtaGroup<CTAS>{});
+    tmem_relinquish(CtaGroup<CTAS>{});
   }
   if constexpr (MODE == kDuoMatched) {
     // Worked out once, as in the roles it took registers from the KV loop.  An odd number of pairs is matched over two slices.
@@ -379,7 +379,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   auto leader = [&](uint64_t* bar) { return CTAS == 2 ? mapa_shared(smem_u32(bar), 0) : smem_u32(bar); };
   if (!SPLIT && dead) {
-    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols, CtaGroup<CTAS>{});
     return;
   }
   const int idx_end = SPLIT && dead ? 0 : total;
@@ -824,7 +824,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync_all();  // neither CTA leaves while the other may still signal it
-  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols, CtaGroup<CTAS>{});
   if constexpr (SPLIT) {
     __syncwarp();
     cluster_sync_all();  // shared memory stays until every CTA has read it

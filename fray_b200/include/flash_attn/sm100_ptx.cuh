@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 // 16-bit operand type of this translation unit: fp16 by default, bf16 when bf16_operands.cuh was
 // included first (the JIT does that for bf16 tensors; every built library has one operand type).
 #ifdef FRAY_ATTN_BF16
@@ -251,16 +253,32 @@ __device__ __forceinline__ void tma_store_wait_read() {
 }
 
 // ---------------------------------------------------------------- TMEM management
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot_in_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)),
-               "r"(ncols)
-               : "memory");
+// CtaGroup<2>: of both CTAs of a pair together, one warp of each (all tcgen05 instructions of a kernel name one cta_group).
+// Allocation and release may wait for the peer's: neither CTA leaves in between, and both get the same columns.
+template <int CTAS>
+using CtaGroup = std::integral_constant<int, CTAS>;
+template <int CTAS = 1>
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot_in_smem, uint32_t ncols, CtaGroup<CTAS> = {}) {
+  if constexpr (CTAS == 1)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)), "r"(ncols)
+                 : "memory");
+  else
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)), "r"(ncols)
+                 : "memory");
 }
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+template <int CTAS = 1>
+__device__ __forceinline__ void tmem_relinquish(CtaGroup<CTAS> = {}) {
+  if constexpr (CTAS == 1)
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  else
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+template <int CTAS = 1>
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols, CtaGroup<CTAS> = {}) {
+  if constexpr (CTAS == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before_sync() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

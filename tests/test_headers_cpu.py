@@ -1,5 +1,6 @@
 """Every kernel header brings in what it uses: each compiles as the only one of a translation unit."""
 import os
+import re
 from concurrent.futures import ThreadPoolExecutor
 
 from fray_b200.jit import build, generate
@@ -18,3 +19,22 @@ def test_each_header_compiles_alone(tmp_path, monkeypatch):
     assert "fwd_split_sm100.cuh" in headers
     with ThreadPoolExecutor() as pool:
         list(pool.map(alone, headers))
+
+
+def test_a_kernel_names_one_cta_group():
+    """All tcgen05 instructions of a kernel have to name the same cta_group: in kernels that are built for one CTA and for pairs
+    each wrapper of one goes by the kernel's number of CTAs, in the others none does."""
+    pairs = 0
+    for header in sorted(os.listdir(HEADERS)):
+        text = re.sub(r"//.*", "", open(os.path.join(HEADERS, header)).read())
+        if header == "sm100_ptx.cuh" or "tmem_alloc" not in text:
+            continue
+        calls = re.findall(r"\b((?:tmem_alloc|tmem_relinquish|tmem_dealloc|mma_ss|mma_ts|mma_commit)\w*[<(][^;]*;)", text)
+        by_argument = ["CtaGroup<CTAS>{}" in call or re.match(r"\w+<CTAS>\(", call) is not None for call in calls]
+        if "int CTAS" in text:
+            pairs += 1
+            assert all(by_argument), (header, calls)
+        else:
+            assert not any(by_argument), (header, calls)
+        assert len(calls) >= 6, header
+    assert pairs == 2
