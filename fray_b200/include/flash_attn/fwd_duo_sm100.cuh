@@ -127,7 +127,9 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool p) {
 // p_bar: the first chunk's barrier, by pointer or by its cluster-wide address (of a pair, the leader's).
 // my_max: this thread's slot for the exchange of maxima, the other half's is other_off floats away; pair_bar: the named
 // barrier of the two warps that share the rows; lim (MASK): keys from lim on are past the end or above the diagonal.
-template <bool MASK, class Bar, class Rescale>
+// MOVE_ALL: when a row's offset has to move, the warp's other rows move theirs to their maxima too, as O is read and written for all 32
+// anyway: fewer steps then have a row whose offset has to move.
+template <bool MASK, bool MOVE_ALL, class Bar, class Rescale>
 __device__ __forceinline__ void softmax_half(uint32_t t_s, Bar p_bar, float* my_max, int other_off, int pair_bar,
                                              Rescale&& rescale_o, int lim, float scale_log2, int lane,
                                              float& m_ref, float& l_run) {
@@ -157,7 +159,7 @@ __device__ __forceinline__ void softmax_half(uint32_t t_s, Bar p_bar, float* my_
     named_barrier_sync(pair_bar, 64);
     const float m_new = max3(mine, my_max[other_off], m_ref);
     float alpha = 1.f;
-    if ((m_new - m_ref) * scale_log2 > kRescaleThreshold) {
+    if (MOVE_ALL ? m_new > m_ref : (m_new - m_ref) * scale_log2 > kRescaleThreshold) {
       // a row without any offset yet has nothing in O (its first product overwrites it)
       alpha = m_ref == -INFINITY ? 1.f : ex2_approx((m_ref - m_new) * scale_log2);
       l_run *= alpha;
@@ -405,17 +407,34 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     float* my_stat = stats + (i * 2 + hf) * 128 + r;
     const int other_off = hf ? -128 : 128;
     const int pair_bar = 1 + i * 4 + (warp & 3);
+    // In a pair a row that moves its offset holds up 16 warps instead of 8: with wide scores, where one does in most steps, pairs with
+    // the code of single CTAs lost 3 % by rows and 2 % by heads to single CTAs.  So all rows of the warp move at a time and O goes
+    // through registers in two pieces; its stores are waited for with those of P (softmax_half).  us, single CTAs : pairs as they
+    // were : now, wide scores, behind lasting load: 7 x 8 x 4046 on 6058 752 : 787 : 755, 9 x 12 x 5029 1421 : 1480 : 1431, causal by
+    // heads 9 x 16/2 x 5161 1054 : 1083 : 1049; scores of unit variance level.
     auto rescale_o = [&](float alpha) {
+      if constexpr (CTAS == 2) {
 #pragma unroll 1
-      for (int c = 0; c < D / 2; c += 16) {
-        uint32_t orr[16];
-        tmem_ld_x16(t_o + c, orr);
-        tmem_wait_ld();
+        for (int c = 0; c < D / 2; c += 32) {
+          uint32_t orr[32];
+          tmem_ld_x32(t_o + c, orr);
+          tmem_wait_ld();
 #pragma unroll
-        for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
-        tmem_st_x16(t_o + c, orr);
+          for (int x = 0; x < 32; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+          tmem_st_x32(t_o + c, orr);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < D / 2; c += 16) {
+          uint32_t orr[16];
+          tmem_ld_x16(t_o + c, orr);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+          tmem_st_x16(t_o + c, orr);
+        }
+        tmem_wait_st();
       }
-      tmem_wait_st();
     };
     // phase parities, toggled: bit 0 s_full, bit 1 o_full, bit 2 stage_free
     uint32_t phases = 0;
@@ -442,13 +461,13 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int j = 0; j < n_full; ++j) {
         wait_scores(j);
         tc_fence_after_sync();
-        softmax_half<false>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, 0, scale_log2, lane, m_ref, l_run);
+        softmax_half<false, CTAS == 2>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, 0, scale_log2, lane, m_ref, l_run);
         phases ^= 1u;
       }
       for (int j = n_full; j < n_i; ++j, lim -= BN) {
         wait_scores(j);
         tc_fence_after_sync();
-        softmax_half<true>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, lim, scale_log2, lane, m_ref, l_run);
+        softmax_half<true, CTAS == 2>(t_s, p_bar, my_stat, other_off, pair_bar, rescale_o, lim, scale_log2, lane, m_ref, l_run);
         phases ^= 1u;
       }
       // The slots carried maxima up to the last step, whose exchange ends with a read of the partner's: both warps have to
@@ -898,6 +917,9 @@ inline bool duo_may_split(int items, int steps, int sms) { return 2 * items <= s
 // causal, by heads: 2 x 32/8 x 3000 164 -> 161, 4 x 40/20 x 2895 411 -> 389, 9 x 40/20 x 1741 358 -> 345; of 71 drawn calls that
 // the rule takes 0.946 to 0.992 times as long.  What it leaves:
 //   * items of 512 rows that need more rounds (1 x 40 x 2610: 1.14, 5 x 40 x 1130: 1.08; by heads they never do);
+//   * items that leave more than a quarter of the last rounds' places empty: the board is not at its limit then, and with wide scores
+//     (see rescale_o) pairs lose 3 to 7 % (1 x 8 x 6031 195 -> 206 us, unit variance 169 -> 168).  With fewer places empty, of 84
+//     drawn calls: unit variance 0.98 by rows and 0.99 by heads, wide scores 1.017 and 0.995 on average (1.00 to 1.03, 0.98 to 1.03);
 //   * fewer than 48 steps of two tiles per SM, or items of fewer than 8 steps (16 x 40 x 3490 on 116 keys: 1.06);
 //   * causal items by rows, whose second pair of tiles works alone for two steps instead of one (4 x 32 x 4096 534 -> 552).
 enum DuoPair : int { kDuoSingle = 0, kDuoPairRows = 1, kDuoPairHeads = 2 };
@@ -907,7 +929,9 @@ inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int ste
   const long long items = static_cast<long long>(slices) * ((seq_len + 255) / 256);
   const long long pair_items = heads ? items / 2 : static_cast<long long>(slices) * ((seq_len + 511) / 512);
   const int pairs = sms / 2;
-  if (pairs <= 0 || (pair_items + pairs - 1) / pairs > (items + sms - 1) / sms) return kDuoSingle;
+  if (pairs <= 0) return kDuoSingle;
+  const long long rounds = (pair_items + pairs - 1) / pairs;
+  if (rounds > (items + sms - 1) / sms || 3 * rounds * pairs > 4 * pair_items) return kDuoSingle;
   if (items * (causal ? (steps + 1) / 2 : steps) < 48LL * sms) return kDuoSingle;
   return heads ? kDuoPairHeads : kDuoPairRows;
 }

@@ -34,6 +34,13 @@ def test_calls_the_rule_leaves(pair):
     assert pair(0, 32, 1, 2048, 16, 148) == SINGLE   # 28 steps per SM: level, and 1.01 on a cooler board
 
 
+def test_calls_whose_last_round_is_mostly_empty(pair):
+    assert pair(0, 12, 1, 6958, 55, 148) == ROWS     # 168 items of 512 rows on three times 74 pairs
+    assert pair(0, 16, 1, 4894, 39, 148) == SINGLE   # 160: 1.015 with wide scores
+    assert pair(0, 8, 1, 6031, 48, 148) == SINGLE    # 96 on twice 74: 1.05
+    assert pair(0, 8, 2, 5861, 46, 148) == SINGLE    # the same by heads, 92: 1.04
+
+
 def test_pairs_never_need_more_rounds(pair):
     for slices in range(2, 400, 2):
         for seq_len in (200, 256, 257, 512, 513, 700, 1024, 1100):
