@@ -124,4 +124,16 @@ inline int flash_attn_pair(const AttnLayout& l) {
   return 0;
 }
 
+// Whether a launch of this layout on the current device runs four independent streams per CTA (1), or a negative AttnReturnCode.
+template <int KIND, int D, int STAGES>
+inline int flash_attn_four_streams(const AttnLayout& l) {
+  if constexpr (KIND == kAttnDuo || KIND == kAttnPersistent) {
+    sm100::DuoPlan plan;
+    const int rc = sm100::duo_plan<D, STAGES>(AttnShape{l.batch_size, l.num_heads, l.seq_len, D},
+                                              AttnShape{l.batch_size, l.num_kv_heads, l.seq_len_kv, D}, l.causal != 0, nullptr, plan);
+    return rc == kAttnOk ? plan.quad : -rc;
+  }
+  return 0;
+}
+
 }  // namespace fray

@@ -946,17 +946,18 @@ inline bool duo_quad(bool causal, long long items, int seq_k, int sms) {
   return causal || !whole_steps || seq_k > 1024 || 2 * items < 5LL * sms;
 }
 
-// How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit).
+// How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit); quad: four independent streams per CTA (head dim 64).
 struct DuoPlan {
   DuoMode mode;
   DuoPair pair;
+  bool quad;
   int parts, sms, items, n_pairs, n_kv;
 };
 
 template <int D, int STAGES>
 inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, cudaStream_t stream, DuoPlan& plan) {
   using Cfg = DuoCfg<D, STAGES>;
-  plan = DuoPlan{kDuoDealt, kDuoSingle, 1, device_sm_count(), 0, 0, 0};
+  plan = DuoPlan{kDuoDealt, kDuoSingle, false, 1, device_sm_count(), 0, 0, 0};
   if (plan.sms <= 0) return kAttnLaunchFailed;
   plan.n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
   plan.n_kv = (shp_kv.S + Cfg::BN - 1) / Cfg::BN;
@@ -974,7 +975,9 @@ inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, 
     if (plan.parts > 1) plan.mode = kDuoSplit;
   } else {
     int units = plan.sms, max_deal = Cfg::kMaxDeal;
-    if constexpr (D == 128) {
+    if constexpr (D == 64) {
+      plan.quad = duo_quad(causal, plan.items, shp_kv.S, plan.sms);
+    } else {
       plan.pair = duo_pair(causal, shp.B * shp.H, shp.H / shp_kv.H, shp.S, steps, plan.sms);
       if (plan.pair != kDuoSingle) {
         if (plan.pair == kDuoPairRows) plan.n_pairs = (shp.S + 4 * Cfg::BM - 1) / (4 * Cfg::BM);
@@ -1039,7 +1042,7 @@ inline int launch_attn_fwd_duo(const operand_t* q, const operand_t* k, const ope
   }
   const bool heaviest_first = duo_heaviest_first(causal, shp, shp_kv);
   if constexpr (D == 64) {
-    if (duo_quad(causal, plan.items, shp_kv.S, plan.sms))
+    if (plan.quad)
       return launch_attn_fwd_quad<D>(tm_q, tm_k, tm_v, tm_o, shp, ex, causal, scale_log2, heaviest_first, plan.mode == kDuoMatched,
                                      plan.n_pairs, plan.items, plan.sms, stream);
     return launch_duo_dealt<D, STAGES, kDuoDealt, 1>(plan, stream, tm_q, tm_k, tm_v, tm_o, shp, ex, causal, scale_log2, heaviest_first);

@@ -54,6 +54,9 @@ extern "C" EXPORT_API int fray_attn_form(const fray::AttnLayout* l, int* mode, i
     return fray::flash_attn_form<{KIND}, {D}, {STAGES}>(*l, mode, parts);
 }
 extern "C" EXPORT_API int fray_attn_pair(const fray::AttnLayout* l) { return fray::flash_attn_pair<{KIND}, {D}, {STAGES}>(*l); }
+extern "C" EXPORT_API int fray_attn_four_streams(const fray::AttnLayout* l) {
+    return fray::flash_attn_four_streams<{KIND}, {D}, {STAGES}>(*l);
+}
 #ifdef FRAY_ATTN_TRACE
 extern "C" EXPORT_API int fray_attn_trace_read(unsigned int* out, int max_words) {
     return fray::sm100::read_attn_trace(out, max_words);

@@ -115,6 +115,19 @@ def test_calls_in_front_of_and_behind_the_other_forms_of_the_row_pair_kernel(mod
     compare_chains(made, order, x, rest, role, causal)
 
 
+# At head dim 64 the row-pair kernel's launcher has two kernels: four streams per CTA (300 items of 128 rows above too), and two
+# threads per row for many short items of whole steps.
+@pytest.mark.parametrize("B,H,S,streams", [(3, 100, 128, 1), (4, 100, 256, 0)])
+@pytest.mark.parametrize("role", [0, 1, 2])
+def test_calls_in_front_of_and_behind_both_kernels_of_head_dim_64(B, H, S, streams, role, monkeypatch):
+    made = runtimes(64, monkeypatch)
+    x, *rest = operands(B, H, S, 64)
+    layout = op._AttnLayout(*op._launch_args(x, x, x, x, may_fold=False)[4:], 0, 1.0)
+    assert made[op.KIND_ROW_PAIRS].symbol("fray_attn_four_streams")(ctypes.byref(layout)) == streams
+    order = [op.KIND_ROW_PAIRS] + [a for kind in made for a in (kind, op.KIND_ROW_PAIRS)]
+    compare_chains(made, order, x, rest, role, causal=False)
+
+
 def test_calls_between_torch_kernels_in_a_graph():
     """Through the public op: the operand is written by a torch kernel just before the call, the output read just after it."""
     from fray_b200.jit_kernels import flash_attn_cute, flash_attn_status
