@@ -247,7 +247,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   } else {
     extern __shared__ __align__(1024) uint8_t duo_smem[];
     smem = duo_smem;
-    fits = (smem_u32(smem) & 1023u) == 0;
+    fits = (opaque(smem_u32(smem)) & 1023u) == 0;
   }
   uint8_t* q_smem = smem + Cfg::kOffQ;
   uint8_t* kv_smem = smem + Cfg::kOffKV;

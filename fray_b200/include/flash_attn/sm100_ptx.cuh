@@ -46,7 +46,11 @@ static constexpr long long kWaitLimitCycles = FRAY_WAIT_LIMIT_CYCLES;
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-
+// The same value, of which the compiler knows nothing: a test of what a declaration promises is not decided by the promise.
+__device__ __forceinline__ uint32_t opaque(uint32_t x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -38,3 +38,12 @@ def test_a_kernel_names_one_cta_group():
             assert not any(by_argument), (header, calls)
         assert len(calls) >= 6, header
     assert pairs == 2
+
+
+def test_a_declared_alignment_is_tested_behind_the_compilers_back():
+    """Swizzled tiles need a base of 1024 bytes.  Where the declaration promises it, a plain test of the address is folded to true."""
+    text = open(os.path.join(HEADERS, "fwd_duo_sm100.cuh")).read()
+    declared = re.findall(r"extern __shared__ __align__\(1024\) uint8_t (\w+)\[\];\s*smem = (\w+);\s*fits = ([^;]*);", text)
+    assert len(declared) == text.count("__align__(1024)") == 1
+    name, base, test = declared[0]
+    assert name == base and re.fullmatch(r"\(opaque\(smem_u32\(smem\)\) & 1023u\) == 0", test)
