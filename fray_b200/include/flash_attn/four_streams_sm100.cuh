@@ -556,7 +556,7 @@ inline int launch_attn_fwd_quad(const CUtensorMap& tm_q, const CUtensorMap& tm_k
   const int fewest = (items + Cfg::kMaxItems - 2) / (Cfg::kMaxItems - 1);  // CTAs: their lists hold no more
   return launch_overlapped(kernel, dim3(items < sms ? items : sms > fewest ? sms : fewest), Cfg::kThreads, Cfg::kSmemBytes, stream, tm_q,
                            tm_k, tm_v, tm_o, shp.H, shp.B * shp.H, shp.S, causal ? 1 : 0, scale_log2, ex.kv_group, ex.lse, ex.seq_k,
-                           heaviest_first ? 1 : 0, matched ? 1 : 0, (ex.seq_k + Cfg::BN - 1) / Cfg::BN, n_pairs, items);
+                           heaviest_first ? 1 : 0, matched ? 1 : 0, pieces(ex.seq_k, Cfg::BN), n_pairs, items);
 }
 
 }  // namespace sm100

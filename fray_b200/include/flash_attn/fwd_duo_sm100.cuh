@@ -874,7 +874,7 @@ inline bool duo_heaviest_first(bool causal, const AttnShape& shp, const AttnShap
 // to 1.04 (8 x 12 x 3935 x 128 420 -> 439), and two query heads per K/V head from 5 % on 0.91 to 1.08 (5 x 32 x 6605 x 128
 // 1608 -> 1732).
 inline bool duo_matched(bool causal, const AttnShape& shp, const AttnShape& shp_kv, long long items, int units, int max_deal) {
-  if (!causal || shp.S <= 1024 || shp.S > ((shp_kv.S + 127) / 128) * 128 || (items & 1) != 0 || items >= (1LL << 30) ||
+  if (!causal || shp.S <= 1024 || shp.S > 128LL * pieces(shp_kv.S, 128) || (items & 1) != 0 || items >= (1LL << 30) ||
       duo_heaviest_first(causal, shp, shp_kv))
     return false;
   const long long twos = items / 2, rounds = (twos + units - 1) / units;
@@ -926,8 +926,8 @@ enum DuoPair : int { kDuoSingle = 0, kDuoPairRows = 1, kDuoPairHeads = 2 };
 inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int steps, int sms) {
   const bool heads = group % 2 == 0;
   if ((causal && !heads) || steps < 8) return kDuoSingle;
-  const long long items = static_cast<long long>(slices) * ((seq_len + 255) / 256);
-  const long long pair_items = heads ? items / 2 : static_cast<long long>(slices) * ((seq_len + 511) / 512);
+  const long long items = static_cast<long long>(slices) * pieces(seq_len, 256);
+  const long long pair_items = heads ? items / 2 : static_cast<long long>(slices) * pieces(seq_len, 512);
   const int pairs = sms / 2;
   if (pairs <= 0) return kDuoSingle;
   const long long rounds = (pair_items + pairs - 1) / pairs;
@@ -942,7 +942,7 @@ inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int ste
 // end of an item, which adds up two accumulators, weighs more than its finer steps gain: 16 x 16 x 1024 with large logits 113 : 110
 // us, 32 x 16 x 512 62.9 : 61.9, 256 keys 39.1 : 38.3, 511 rows on 194 keys 23.7 : 22.7; 1280 keys 122.1 : 122.6.
 inline bool duo_quad(bool causal, long long items, int seq_k, int sms) {
-  const bool whole_steps = (seq_k + 63) / 64 % 2 == 0;  // the last 128 keys are more than half there
+  const bool whole_steps = pieces(seq_k, 64) % 2 == 0;  // the last 128 keys are more than half there
   return causal || !whole_steps || seq_k > 1024 || 2 * items < 5LL * sms;
 }
 
@@ -959,8 +959,8 @@ inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, 
   using Cfg = DuoCfg<D, STAGES>;
   plan = DuoPlan{kDuoDealt, kDuoSingle, false, 1, device_sm_count(), 0, 0, 0};
   if (plan.sms <= 0) return kAttnLaunchFailed;
-  plan.n_pairs = (shp.S + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
-  plan.n_kv = (shp_kv.S + Cfg::BN - 1) / Cfg::BN;
+  plan.n_pairs = pieces(shp.S, 2 * Cfg::BM);
+  plan.n_kv = pieces(shp_kv.S, Cfg::BN);
   plan.items = plan.n_pairs * shp.B * shp.H;
   const int steps = causal && 2 * plan.n_pairs < plan.n_kv ? 2 * plan.n_pairs : plan.n_kv;
   if (duo_may_split(plan.items, steps, plan.sms)) {
@@ -980,7 +980,7 @@ inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, 
     } else {
       plan.pair = duo_pair(causal, shp.B * shp.H, shp.H / shp_kv.H, shp.S, steps, plan.sms);
       if (plan.pair != kDuoSingle) {
-        if (plan.pair == kDuoPairRows) plan.n_pairs = (shp.S + 4 * Cfg::BM - 1) / (4 * Cfg::BM);
+        if (plan.pair == kDuoPairRows) plan.n_pairs = pieces(shp.S, 4 * Cfg::BM);
         plan.items = plan.n_pairs * shp.B * shp.H / (plan.pair == kDuoPairHeads ? 2 : 1);
         units = plan.sms / 2;
         max_deal = DuoCfg<D, STAGES, 2>::kMaxDeal;

@@ -281,6 +281,9 @@ inline int heaviest_first_group(bool causal, const AttnShape& shp, const AttnSha
   return heaviest_first_order(causal, shp, shp_kv) ? shp.B * shp.H : 0;
 }
 
+// Pieces of `size` that `n` rows take (n up to the largest int, where n + size - 1 would wrap).
+inline int pieces(int n, int size) { return n / size + (n % size != 0); }
+
 // Number of SMs of the current device (cached per device of this process); 0 on failure.
 inline int device_sm_count() {
   constexpr int kMaxDevices = 64;

@@ -41,6 +41,12 @@ def test_calls_whose_last_round_is_mostly_empty(pair):
     assert pair(0, 8, 2, 5861, 46, 148) == SINGLE    # the same by heads, 92: 1.04
 
 
+def test_the_longest_folded_sequences(pair):
+    longest = 2 ** 31 - 1 - 255  # what folded groups may grow to
+    for seq_len in (longest - 256, longest, 2 ** 31 - 1):
+        assert pair(0, 2, 1, seq_len, 8, 148) == ROWS and pair(0, 2, 2, seq_len, 8, 148) == HEADS
+
+
 def test_pairs_never_need_more_rounds(pair):
     for slices in range(2, 400, 2):
         for seq_len in (200, 256, 257, 512, 513, 700, 1024, 1100):
