@@ -923,17 +923,20 @@ inline bool duo_may_split(int items, int steps, int sms) { return 2 * items <= s
 //   * fewer than 48 steps of two tiles per SM, or items of fewer than 8 steps (16 x 40 x 3490 on 116 keys: 1.06);
 //   * causal items by rows, whose second pair of tiles works alone for two steps instead of one (4 x 32 x 4096 534 -> 552).
 enum DuoPair : int { kDuoSingle = 0, kDuoPairRows = 1, kDuoPairHeads = 2 };
-inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int steps, int sms) {
+// pairs: that run at the same time.
+inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int steps, int sms, int pairs) {
   const bool heads = group % 2 == 0;
   if ((causal && !heads) || steps < 8) return kDuoSingle;
   const long long items = static_cast<long long>(slices) * pieces(seq_len, 256);
   const long long pair_items = heads ? items / 2 : static_cast<long long>(slices) * pieces(seq_len, 512);
-  const int pairs = sms / 2;
   if (pairs <= 0) return kDuoSingle;
   const long long rounds = (pair_items + pairs - 1) / pairs;
   if (rounds > (items + sms - 1) / sms || 3 * rounds * pairs > 4 * pair_items) return kDuoSingle;
   if (items * (causal ? (steps + 1) / 2 : steps) < 48LL * sms) return kDuoSingle;
   return heads ? kDuoPairHeads : kDuoPairRows;
+}
+inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int steps, int sms) {
+  return duo_pair(causal, slices, group, seq_len, steps, sms, sms / 2);
 }
 
 // Head dim 64: whether the items go to the kernel with four independent streams per CTA (four_streams_sm100.cuh) instead.  Of
@@ -946,19 +949,33 @@ inline bool duo_quad(bool causal, long long items, int seq_k, int sms) {
   return causal || !whole_steps || seq_k > 1024 || 2 * items < 5LL * sms;
 }
 
-// How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit); quad: four independent streams per CTA (head dim 64).
+// How a problem is dealt to the CTAs; parts: CTAs per item (kDuoSplit); quad: four independent streams per CTA (head dim 64);
+// units: CTAs, or CTA pairs, that run at the same time.
 struct DuoPlan {
   DuoMode mode;
   DuoPair pair;
   bool quad;
-  int parts, sms, items, n_pairs, n_kv;
+  int parts, sms, units, items, n_pairs, n_kv;
 };
+
+// CTA pairs that run at the same time: half of the SMs, unless the device or its share of one places fewer; 0 on failure.
+template <int D, int STAGES>
+inline int duo_pairs_at_a_time(int sms, cudaStream_t stream) {
+  using Cfg = DuoCfg<D, STAGES, 2>;
+  auto kernel = attn_fwd_duo_kernel<D, STAGES, kDuoDealt, 2>;
+  struct Tag {};
+  if (ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal) != kAttnOk) return 0;
+  ClusterLaunch launch(1, Cfg::kThreads, Cfg::kSmemBytes, stream);
+  const auto* active = active_cluster_counts<Tag>(kernel, launch);
+  return active == nullptr ? 0 : (*active)[2] < sms / 2 ? (*active)[2] : sms / 2;
+}
 
 template <int D, int STAGES>
 inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, cudaStream_t stream, DuoPlan& plan) {
   using Cfg = DuoCfg<D, STAGES>;
-  plan = DuoPlan{kDuoDealt, kDuoSingle, false, 1, device_sm_count(), 0, 0, 0};
+  plan = DuoPlan{kDuoDealt, kDuoSingle, false, 1, device_sm_count(), 0, 0, 0, 0};
   if (plan.sms <= 0) return kAttnLaunchFailed;
+  plan.units = plan.sms;
   plan.n_pairs = pieces(shp.S, 2 * Cfg::BM);
   plan.n_kv = pieces(shp_kv.S, Cfg::BN);
   plan.items = plan.n_pairs * shp.B * shp.H;
@@ -974,19 +991,23 @@ inline int duo_plan(const AttnShape& shp, const AttnShape& shp_kv, bool causal, 
     plan.parts = duo_parts(plan.items, steps, causal, plan.sms, *active);
     if (plan.parts > 1) plan.mode = kDuoSplit;
   } else {
-    int units = plan.sms, max_deal = Cfg::kMaxDeal;
+    int max_deal = Cfg::kMaxDeal;
     if constexpr (D == 64) {
       plan.quad = duo_quad(causal, plan.items, shp_kv.S, plan.sms);
     } else {
       plan.pair = duo_pair(causal, shp.B * shp.H, shp.H / shp_kv.H, shp.S, steps, plan.sms);
       if (plan.pair != kDuoSingle) {
+        const int pairs = duo_pairs_at_a_time<D, STAGES>(plan.sms, stream);
+        plan.pair = duo_pair(causal, shp.B * shp.H, shp.H / shp_kv.H, shp.S, steps, plan.sms, pairs);
+        if (plan.pair != kDuoSingle) plan.units = pairs;
+      }
+      if (plan.pair != kDuoSingle) {
         if (plan.pair == kDuoPairRows) plan.n_pairs = pieces(shp.S, 4 * Cfg::BM);
         plan.items = plan.n_pairs * shp.B * shp.H / (plan.pair == kDuoPairHeads ? 2 : 1);
-        units = plan.sms / 2;
         max_deal = DuoCfg<D, STAGES, 2>::kMaxDeal;
       }
     }
-    if (duo_matched(causal, shp, shp_kv, plan.items, units, max_deal)) plan.mode = kDuoMatched;  // two items per SM and more
+    if (duo_matched(causal, shp, shp_kv, plan.items, plan.units, max_deal)) plan.mode = kDuoMatched;  // two items per SM and more
   }
   return kAttnOk;
 }
@@ -1000,8 +1021,7 @@ inline int launch_duo_dealt(const DuoPlan& plan, cudaStream_t stream, const CUte
   struct Tag {};
   const int rc = ensure_dynamic_smem<Tag>(kernel, Cfg::kSmemBytes, Cfg::kThreads, Cfg::kRegsTotal);
   if (rc != kAttnOk) return rc;
-  const int units = plan.sms / CTAS;
-  const int clusters = plan.items < units ? plan.items : units;
+  const int clusters = plan.items < plan.units ? plan.items : plan.units;
   auto launch = [&](auto... args) {
     if constexpr (CTAS == 1) return launch_overlapped(kernel, dim3(clusters), Cfg::kThreads, Cfg::kSmemBytes, stream, args...);
     ClusterLaunch cluster(clusters, Cfg::kThreads, Cfg::kSmemBytes, stream);

@@ -41,6 +41,20 @@ def test_calls_whose_last_round_is_mostly_empty(pair):
     assert pair(0, 8, 2, 5861, 46, 148) == SINGLE    # the same by heads, 92: 1.04
 
 
+def test_fewer_pairs_than_half_of_the_sms(pair, monkeypatch):
+    from fray_b200.jit import build, generate
+    args = (("n", int),)
+    code = generate(op.includes, args, "\n__return_code = 0;\n", """
+extern "C" EXPORT_API int pair(int slices, int group, int seq_len, int steps, int sms, int pairs) {
+    return fray::sm100::duo_pair(false, slices, group, seq_len, steps, sms, pairs);
+}
+""")
+    of = build("pair_rule_places", args, code).symbol("pair")
+    assert of(128, 1, 4096, 32, 148, 74) == ROWS and of(128, 1, 4096, 32, 148, 73) == SINGLE  # 1024 items on 73: 15 rounds for 14
+    assert of(128, 2, 4096, 32, 148, 74) == HEADS and of(128, 2, 4096, 32, 148, 70) == SINGLE
+    assert of(128, 1, 4096, 32, 148, 0) == SINGLE  # a device that places none
+
+
 def test_the_longest_folded_sequences(pair):
     longest = 2 ** 31 - 1 - 255  # what folded groups may grow to
     for seq_len in (longest - 256, longest, 2 ** 31 - 1):
