@@ -89,10 +89,12 @@ struct DuoCfg {
   static constexpr int kNumBars = 2 * 2 + 2 * kRing + 2 * 3 + 2 * kPChunks + 4;
   static constexpr int kOffStats = kOffBars + ((kNumBars * 8 + 16 + 127) / 128) * 128;  // [2 tiles][2 halves][128]
   static constexpr int kOffDeal = kOffStats + 4 * 128 * 4;
-  // kDuoMatched: a CTA's items and the end mark, as many as shared memory has room for at head dim 128 and four slots: 189 items
-  // a CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048).  Causal problems of more items are dealt slice by slice.
+  // kDuoMatched (head dim 128): a CTA's items and the end mark, as many as shared memory has room for with four slots: 189 items a
+  // CTA, 28 000 on 148 SMs (4 x 32 x 4096 has 2048), and 139 a pair.  Causal problems of more items are dealt slice by slice, at head
+  // dim 64, too, where four streams deal by lists of their own: matched is level there (us, 28 000 to 37 000 items, slice by slice :
+  // matched: 80 x 80 x 1280 2471 : 2473, 50 x 80 x 2048 3459 : 3464, 60 x 80/40 x 1792 3223 : 3188, 40 x 50 x 4096 6061 : 6096).
   static constexpr int kMaxDeal = CTAS == 2 ? 140 : 190;
-  static constexpr int kUsedBytes = kOffDeal + kMaxDeal * 4;
+  static constexpr int kUsedBytes = kOffDeal + (D == 128 ? kMaxDeal * 4 : 0);
   // slack for the forms that bring the dynamic segment to a 1024-byte boundary themselves (its base is one already; checked)
   static constexpr int kSmemBytes = kUsedBytes + 1024 <= 232448 ? kUsedBytes + 1024 : 232448;
   static_assert(kUsedBytes <= 232448, "exceeds the 227 KB shared memory of one CTA");
@@ -233,6 +235,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   constexpr int RING = Cfg::kRing;
   constexpr bool SPLIT = MODE == kDuoSplit;
   static_assert(CTAS == 1 || !SPLIT, "a split item's clusters are of single CTAs");
+  static_assert(MODE != kDuoMatched || D == 128, "head dim 64 has no room for a deal: four streams match its items");
   uint8_t* smem;
   bool fits;
   // Aligned by declaration every address in it is a constant, which the long items of the matched form and of pairs gain 1 % by
