@@ -143,14 +143,8 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   int4* items = reinterpret_cast<int4*>(smem + Cfg::kOffItems);
   for (int k = tid - 64; k >= 0 && k < Cfg::kMaxItems; k += Cfg::kThreads - 64) {
     int idx;
-    if (matched) {  // an odd number of pairs is matched over two slices
-      const int two = n_pairs & 1, run = n_pairs << two;
-      const int d = (k >> 1) * stride + unit;
-      const int group = 2 * d / run, j = d - group * (run >> 1), r = (k & 1) ? run - 1 - j : j;
-      idx = 2 * d < total ? ((group << two) + (r & two)) * n_pairs + (r >> two) : total;
-    } else {
-      idx = k * stride + ((causal && (k & 1)) ? stride - 1 - unit : unit);
-    }
+    if (matched) idx = matched_item(k, stride, unit, n_pairs, total);
+    else idx = k * stride + ((causal && (k & 1)) ? stride - 1 - unit : unit);
     int4 item = make_int4(-1, 0, 0, 0);
     if (idx < total) {
       const int run = heaviest_first ? num_bh : n_pairs;
@@ -208,15 +202,7 @@ attn_fwd_quad_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           if (c + 32 >= lim) sb[c] = __float_as_uint(-INFINITY);
         }
       }
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 32; c += 4) {
-        mx0 = max3(mx0, __uint_as_float(sa[c + 0]), __uint_as_float(sb[c + 0]));
-        mx1 = max3(mx1, __uint_as_float(sa[c + 1]), __uint_as_float(sb[c + 1]));
-        mx2 = max3(mx2, __uint_as_float(sa[c + 2]), __uint_as_float(sb[c + 2]));
-        mx3 = max3(mx3, __uint_as_float(sa[c + 3]), __uint_as_float(sb[c + 3]));
-      }
-      const float mine = fmaxf(max3(mx0, mx1, mx2), mx3);
+      const float mine = max_64(sa, sb);
       if (__any_sync(0xffffffffu, (mine - m_ref) * scale_log2 > kRescaleThreshold)) {
         float alpha = 1.f;
         if ((mine - m_ref) * scale_log2 > kRescaleThreshold) {

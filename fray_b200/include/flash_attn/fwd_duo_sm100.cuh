@@ -147,15 +147,7 @@ __device__ __forceinline__ void softmax_half(uint32_t t_s, Bar p_bar, float* my_
       if (c + 32 >= lim) sb[c] = __float_as_uint(-INFINITY);
     }
   }
-  float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-  for (int c = 0; c < 32; c += 4) {
-    mx0 = max3(mx0, __uint_as_float(sa[c + 0]), __uint_as_float(sb[c + 0]));
-    mx1 = max3(mx1, __uint_as_float(sa[c + 1]), __uint_as_float(sb[c + 1]));
-    mx2 = max3(mx2, __uint_as_float(sa[c + 2]), __uint_as_float(sb[c + 2]));
-    mx3 = max3(mx3, __uint_as_float(sa[c + 3]), __uint_as_float(sb[c + 3]));
-  }
-  const float mine = fmaxf(max3(mx0, mx1, mx2), mx3);
+  const float mine = max_64(sa, sb);
   if (named_barrier_or(pair_bar, 64, (mine - m_ref) * scale_log2 > kRescaleThreshold)) {
     *my_max = mine;
     named_barrier_sync(pair_bar, 64);
@@ -359,13 +351,9 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tmem_relinquish(CtaGroup<CTAS>{});
   }
   if constexpr (MODE == kDuoMatched) {
-    // Worked out once, as in the roles it took registers from the KV loop.  An odd number of pairs is matched over two slices.
-    const int two = n_pairs & 1, run = n_pairs << two;
-    for (int k = tid - 64; k >= 0 && k < Cfg::kMaxDeal; k += Cfg::kThreads - 64) {
-      const int d = (k >> 1) * stride + unit;
-      const int group = 2 * d / run, j = d - group * (run >> 1), r = (k & 1) ? run - 1 - j : j;
-      reinterpret_cast<uint32_t*>(smem + Cfg::kOffDeal)[k] = 2 * d < total ? ((group << two) + (r & two)) * n_pairs + (r >> two) : total;
-    }
+    // worked out once, as in the roles it took registers from the KV loop
+    for (int k = tid - 64; k >= 0 && k < Cfg::kMaxDeal; k += Cfg::kThreads - 64)
+      reinterpret_cast<uint32_t*>(smem + Cfg::kOffDeal)[k] = matched_item(k, stride, unit, n_pairs, total);
   }
   grid_dependency_wait();
   if (tid == 32) *abort_flag = (*reinterpret_cast<volatile int*>(&fray_attn_status[0]) != 0) ? 2u : 0u;

@@ -78,6 +78,28 @@ inline int read_attn_trace(unsigned int* out, int max_words) {
 // Lazy-rescale threshold in the scaled base-2 domain: offsets move only when the max grew by > 2^8.
 static constexpr float kRescaleThreshold = 8.0f;
 
+// Largest of 64 scores.
+__device__ __forceinline__ float max_64(const uint32_t (&sa)[32], const uint32_t (&sb)[32]) {
+  float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    mx0 = max3(mx0, __uint_as_float(sa[c + 0]), __uint_as_float(sb[c + 0]));
+    mx1 = max3(mx1, __uint_as_float(sa[c + 1]), __uint_as_float(sb[c + 1]));
+    mx2 = max3(mx2, __uint_as_float(sa[c + 2]), __uint_as_float(sb[c + 2]));
+    mx3 = max3(mx3, __uint_as_float(sa[c + 3]), __uint_as_float(sb[c + 3]));
+  }
+  return fmaxf(max3(mx0, mx1, mx2), mx3);
+}
+
+// Item number k of CTA (CTA pair) `unit` of `stride`, matched by twos: an item and the one of its slice that has as many steps less
+// than the middle as it has more; an odd number of pairs of tiles to a slice is matched over two slices.  `total`: there is none.
+__device__ __forceinline__ int matched_item(int k, int stride, int unit, int n_pairs, int total) {
+  const int two = n_pairs & 1, run = n_pairs << two;
+  const int d = (k >> 1) * stride + unit;
+  const int group = 2 * d / run, j = d - group * (run >> 1), r = (k & 1) ? run - 1 - j : j;
+  return 2 * d < total ? ((group << two) + (r & two)) * n_pairs + (r >> two) : total;
+}
+
 // 32 keys of one row: exponentials in base 2 of scale * score - offset, row sum from the unrounded values (two packed
 // partial sums), rounding to 16 bits.
 __device__ __forceinline__ void exp_32(const uint32_t (&h)[32], uint64_t scale2, uint64_t neg_m2, uint64_t& rsp0,
