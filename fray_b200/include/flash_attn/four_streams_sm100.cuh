@@ -27,6 +27,8 @@
 // us, two threads per row -> four streams, each behind lasting load: 6 x 12 x 333 causal 8.9 -> 8.1, 3 x 16/4 x 1326 causal 27.8
 // -> 26.2, 2 x 32/8 x 3000 causal 119.8 -> 115.5, 4 x 16 x 4096 causal 209.5 -> 203.4, 1 x 32 x 16384 causal 1490 -> 1452,
 // 8 x 16 x 4096 725 -> 712, 16 x 16 x 900 with large logits 110.2 -> 105.0.
+// Wide scores, whose offsets move often, two of them per row: 0.81 to 0.97 of the time of two threads per row over 34 drawn calls of
+// up to 8413 keys (unit variance 0.82 to 0.98).  The compiler spills: 88 bytes of stores and 92 of loads at 96 registers.
 // Tried and left out: 12 or 25 % of the exponentials on the FMA pipe (level, 2 to 5 % slower: the board is at its power limit),
 // scores fetched again instead of kept (spills elsewhere, 3 % slower), the merge by the group that ends last while the other goes on
 // (400 bytes of spills, 10 % slower), tile 1 started behind tile 0 (level), offsets moved from 2^12 on instead of 2^8 (level).

@@ -29,7 +29,7 @@
 //     soon as they are in registers, and a warp of its own stores finished tiles from one staging tile that both query
 //     tiles use in turn, which leaves room for four ring slots at head dim 128.
 //   * Values a step does not need are worked out again per item instead of kept: 104 registers hold a half row and its
-//     P without spills (10 % against the first version, which spilled 100 bytes).
+//     P with 4 to 24 bytes of spill stores, by form (10 % against the first version, which spilled 100).
 //
 // Measured against the faster of the two-tile and the one-tile kernel, each behind 150 ms of its own load (us, same run): 4 x
 // 32 x 4096 x 128 981-1028 : 1051-1099, causal 569-572 : 648-656, 1 x 32 x 16384 causal 2070-2080 : 2180-2261, 2 x 16 x 2048 75 :
@@ -232,7 +232,7 @@ attn_fwd_duo_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   bool fits;
   // Aligned by declaration every address in it is a constant, which the long items of the matched form and of pairs gain 1 % by
   // (1 x 32 x 16384 causal 1930 -> 1912 us); short items lose (3 x 32 x 826 on 184 keys 21.8 : 23.6, 6 x 16 x 333 causal 16.8 :
-  // 17.5, split: 2 slices of 264 rows on 1913 keys 15.2 : 15.5), so the other forms round it up here.
+  // 17.5, split: 2 slices of 264 rows on 1913 keys 15.2 : 15.5), so the other forms round it up here.  Why they lose is not known.
   if constexpr (SPLIT || (D == 128 && MODE == kDuoDealt && CTAS == 1)) {
     extern __shared__ uint8_t duo_raw[];
     const uint32_t raw_addr = smem_u32(duo_raw);
@@ -906,7 +906,7 @@ inline bool duo_may_split(int items, int steps, int sms) { return 2 * items <= s
 // the pair's start, end and common pace cost more (behind 15 ms of load instead of 60, up to 120 us: 1.00 to 1.07 times as long).
 // us, single CTAs -> pairs, behind lasting load: 4 x 32 x 4096 993 -> 973, 16 x 16 x 1024 148 -> 147, 2 x 32 x 2325 203 -> 198,
 // causal, by heads: 2 x 32/8 x 3000 164 -> 161, 4 x 40/20 x 2895 411 -> 389, 9 x 40/20 x 1741 358 -> 345; of 71 drawn calls that
-// the rule takes 0.946 to 0.992 times as long.  What it leaves:
+// the rule takes, with scores of unit variance, 0.946 to 0.992 times as long.  What it leaves:
 //   * items of 512 rows that need more rounds (1 x 40 x 2610: 1.14, 5 x 40 x 1130: 1.08; by heads they never do);
 //   * items that leave more than a quarter of the last rounds' places empty: the board is not at its limit then, and with wide scores
 //     (see rescale_o) pairs lose 3 to 7 % (1 x 8 x 6031 195 -> 206 us, unit variance 169 -> 168).  With fewer places empty, of 84
@@ -932,7 +932,7 @@ inline DuoPair duo_pair(bool causal, int slices, int group, int seq_len, int ste
 
 // Head dim 64: whether the items go to the kernel with four independent streams per CTA (four_streams_sm100.cuh) instead.  Of
 // 105 drawn calls that the rule sends there (1 to 46 steps, 80 to 4800 items, with and without a causal mask) it took 0.84 to 1.01
-// times as long, 0.92 on average.  What it loses are many short items that all end with whole steps, where its
+// times as long, 0.92 on average; with wide scores 0.81 to 0.97, 0.92 in the middle (34 calls, up to 8413 keys).  What it loses are many short items that all end with whole steps, where its
 // end of an item, which adds up two accumulators, weighs more than its finer steps gain: 16 x 16 x 1024 with large logits 113 : 110
 // us, 32 x 16 x 512 62.9 : 61.9, 256 keys 39.1 : 38.3, 511 rows on 194 keys 23.7 : 22.7; 1280 keys 122.1 : 122.6.
 inline bool duo_quad(bool causal, long long items, int seq_k, int sms) {

@@ -178,7 +178,7 @@ inline int ensure_dynamic_smem(Kernel kernel, int bytes, int threads = 0, int re
 
 // Launches a kernel whose CTAs may be set up (barriers, tensor memory) while the stream's previous kernel drains; the
 // kernel itself waits for that one's end before it touches global memory (grid_dependency_wait).  Per call, back to back
-// on one stream: 6 x 12 x 333 x 64 causal 12.3 -> 10.9 us, 2 x 16 x 2048 x 128 78.8 -> 77.0, 8 x 8 x 8192 decode
+// on one stream: 6 x 12 x 333 x 64 causal 10.2 -> 8.2 us, 2 x 16 x 2048 x 128 74.6 -> 73.1, 8 x 8 x 8192 decode
 // 52.2 -> 51.3; nothing from 100 us on.
 template <class... Params, class... Args>
 inline int launch_overlapped(void (*kernel)(Params...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, Args... args) {

@@ -250,8 +250,8 @@ def _workload_class(seq_len: int, seq_len_kv: int, units: int, sms: int) -> str:
     """Coarse workload class the tuner memoises on, from what the kinds differ in: how many steps a work item has (bucket of
     the number of keys), whether items of two query tiles fill the chip, and whether there is a second tile at all.  Items for up
     to half of the SMs are apart: an SM for each of their tiles (one-tile kernels), or two and more CTAs for each (row-pair kernel
-    with its keys split).  As one class, the call that came first decided: 146 items of 333 causal rows, head dim 64, 9.0 us, or
-    16.2 behind 4 items; 48 heads of 256 rows on 2048 keys, head dim 128, 20.1, or 27.5 behind 140."""
+    with its keys split).  As one class, the call that came first decided: 144 items of 333 causal rows, head dim 64, 8.2 us, or
+    16.2 behind 4 items; 48 heads of 256 rows on 2048 keys, head dim 128, 20.1, or 25.1 behind 140."""
     k_bucket = 1 << max(7, (max(seq_len_kv, 1) - 1).bit_length())
     items = units * -(-seq_len // 256)
     fill = "big" if items >= sms else "half" if 2 * items <= sms else "small"
